@@ -38,3 +38,21 @@ def test_zero_state_is_refused():
         with pytest.raises(ValueError):
             sv.sample_indices(shots, seed=1)
     sv.close()
+
+
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+@pytest.mark.parametrize("n,wires", [
+    (1, []), (3, []), (3, [2]), (4, [3, 0]), (5, [4, 3, 2, 1]), (6, [5]), (7, [6, 5, 4, 3, 2]), (9, [8, 0, 7]),
+    (10, list(range(1, 10))), (11, list(range(11))[::-1]), (12, [11, 10, 9, 8]), (12, [8, 9]), (13, [12, 3, 10]),
+    (13, list(range(12))), (15, [14, 11, 12, 13, 0, 7]), (17, [3]), (20, [19, 17, 2, 9]), (21, [20]), (22, [])])
+def test_marginals_over_chunk_and_sibling_edges(n, wires, dtype):
+    """Chunks of 1 to 1024 entries (below and above a warp), 0 to 4 selected
+    qubits on the low index bits, one level of sums to three."""
+    vec = rand_state(n, 3 * n + len(wires), dtype)
+    sv = _sv(n, dtype, vec)
+    ref = osamp.marginal_probabilities(osamp.amp2(vec), n, wires)
+    assert np.array_equal(sv.probabilities(wires), ref)
+    assert np.array_equal(sv.probabilities(wires, dtype=np.float32), ref.astype(np.float32))
+    if wires:
+        assert np.array_equal(sv.sample_indices(50, wires, seed=4), osamp.sample_indices(ref, 4, 50))
+    sv.close()
