@@ -3,6 +3,7 @@
 import numpy as np
 import pytest
 
+from oracle import OracleSim
 from oracle import sampler as osamp
 from tests.helpers import rand_state
 
@@ -55,4 +56,34 @@ def test_marginals_over_chunk_and_sibling_edges(n, wires, dtype):
     assert np.array_equal(sv.probabilities(wires, dtype=np.float32), ref.astype(np.float32))
     if wires:
         assert np.array_equal(sv.sample_indices(50, wires, seed=4), osamp.sample_indices(ref, 4, 50))
+    sv.close()
+
+
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+@pytest.mark.parametrize("n", [1, 2, 5, 11, 12, 13, 14, 18, 19, 20, 21])
+def test_pauli_words_over_every_kernel_of_the_split(n, dtype):
+    """Words without X and Y, words within four neighbouring index bits (in
+    every window, with Z letters inside and outside it), and words spread over
+    the register, more of one kind than a launch holds.  Both sides sum the
+    exact float64 products of the same amplitudes: 1e-12 covers the rounding
+    of 2^21 additions of a unit vector's terms."""
+    vec = rand_state(n, 7 * n, dtype)
+    rng = np.random.default_rng(n)
+    words = [{}] + [{q: p} for q in range(n) for p in "XYZ"] + [{q: a, q + 1: b} for q in range(n - 1)
+                                                               for a, b in ("XX", "YY", "ZZ", "XY")]
+    for _ in range(12):
+        lo = int(rng.integers(0, max(1, n - 3)))
+        words.append({q: "XYZ"[int(rng.integers(3))] for q in range(lo, min(n, lo + 4))})
+        words.append({int(q): "XYZ"[int(rng.integers(3))] for q in rng.permutation(n)[:int(rng.integers(1, min(n, 7) + 1))]})
+    if n > 14:
+        words = [words[i] for i in sorted(rng.permutation(len(words))[:60])]
+    sv = _sv(n, dtype, vec)
+    got = sv.expval_pauli(words)
+    o = OracleSim(n, np.complex128)
+    o.set_state(vec.astype(np.complex128))
+    ref = np.array([o.pauli_expectation(w) for w in words])
+    assert np.max(np.abs(got - ref)) < 1e-12
+    assert np.array_equal(sv.expval_pauli(words), got)
+    one = int(rng.integers(len(words)))
+    assert sv.expval_pauli([words[one]])[0] == got[one]  # a word's bits do not depend on the others
     sv.close()
