@@ -363,24 +363,7 @@ int mq_apply_qft(mq_state* h, const int32_t* wires, int k, int inverse) {
   for (int i = 1; i < k; ++i)
     if (wires[i] != wires[0] + i) contiguous = false;
   if (contiguous) return launch_qft_contiguous(h, wires[0], k, inverse);
-  // Move wire j to qubit j (others keep their relative order after them),
-  // run the contiguous QFT on qubits [0, k), and move back.  Wire
-  // permutations are GF(2) linear, so each move is one permutation sweep.
-  std::vector<int> sigma(n, -1);  // old qubit -> new qubit
-  int next = k;
-  for (int j = 0; j < k; ++j) sigma[wires[j]] = j;
-  for (int q = 0; q < n; ++q)
-    if (sigma[q] < 0) sigma[q] = next++;
-  uint32_t fwd[32], back[32];
-  for (int q = 0; q < n; ++q) {
-    fwd[n - 1 - sigma[q]] = 1u << (n - 1 - q);
-    back[n - 1 - q] = 1u << (n - 1 - sigma[q]);
-  }
-  int rc = launch_affine_cols(h, fwd, 0);
-  if (rc) return rc;
-  rc = launch_qft_contiguous(h, 0, k, inverse);
-  if (rc) return rc;
-  return launch_affine_cols(h, back, 0);
+  return launch_qft_wires(h, wires, k, inverse);
   MQ_TRY_END
 }
 

@@ -288,6 +288,7 @@ int take_adj_fault(mq_state* h, bool* fault);
 // Tile sweeps: U(2) layer and QFT (mq_tile.cu)
 int launch_u2_layer(mq_state* h, const double* mats, const uint8_t* active);
 int launch_qft_contiguous(mq_state* h, int q0, int k, int inverse);
+int launch_qft_wires(mq_state* h, const int32_t* wires, int k, int inverse);
 int launch_qft_stages(mq_state* h, int q0, int k, int j_begin, int j_end, int inverse);
 int launch_cu2_list(mq_state* h, int n_gates, const int32_t* targets, const uint32_t* cmasks, const double* mats);
 // Diagonal layers (mq_diag.cu)

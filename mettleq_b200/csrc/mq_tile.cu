@@ -163,9 +163,15 @@ struct FusedParams : TileParams {
 };
 // QFT sweeps: per stage op, the phase factor of each register pattern r
 // (e^{i pi Lr(r) / 2^width}, see apply_qft).
+// lmap: the transform's wires are not one run of index bits.  The twiddles
+// then read the ladder value L itself (wire j of k has weight 2^(k-1-j), other
+// bits none) instead of a shifted index: PhaseDesc g_reg / g_grp hold weights,
+// and L of a tile's base is the XOR of ltab[256 i + byte i of the tile number].
 struct QftParams : TileParams {
   alignas(16) float2 twf[kMaxOps][32];
   alignas(16) double2 twd[kMaxOps][32];
+  uint32_t lmap;
+  uint32_t ltab[1024];
 };
 static_assert(sizeof(QftParams) <= 32000, "kernel parameter block too large");
 static_assert(sizeof(FusedParams) <= 32000, "kernel parameter block too large");
@@ -805,6 +811,13 @@ k_tile(const V2<R>* src, V2<R>* dst, const __grid_constant__ PT P) {
     }
     uint32_t cl_in;
     const uint32_t base = src_base(tile, cl_in);
+    // what a group's global index starts from: the base, or its ladder value
+    uint32_t gbase = base;
+    if constexpr (QFT) {
+      if (P.lmap)
+        gbase = P.ltab[tile & 255u] ^ P.ltab[256 + ((tile >> 8) & 255u)] ^ P.ltab[512 + ((tile >> 16) & 255u)] ^
+                P.ltab[768 + (tile >> 24)];
+    }
     for (int ph = 0; ph < P.n_phases; ++ph) {
       const PhaseDesc& D = phs[ph];
       uint32_t greg[LR], sreg[LR];
@@ -821,7 +834,7 @@ k_tile(const V2<R>* src, V2<R>* dst, const __grid_constant__ PT P) {
         // thread bits from the phase's tables, the bits of g (above LT) from
         // the descriptor (compile-time selected)
         const uint32_t* tt = ttab + ph * kThreadTabWords;
-        uint32_t sq = tt[t_lo] ^ tt[16 + t_hi], gq = base;
+        uint32_t sq = tt[t_lo] ^ tt[16 + t_hi], gq = gbase;
 #pragma unroll
         for (int j = LT; j < M - LR; ++j)
           if ((q >> j) & 1) sq ^= D.s_grp[j];
@@ -1064,6 +1077,10 @@ struct Sweep {
   // rotation matrices may run in tangent form (PhaseDesc::rot); the caller
   // multiplies the product of their factors (rot_factor) into a diagonal
   bool rot = false;
+  // QFT on wires that are not one run of index bits: the ladder weight of every
+  // index bit (0: not a wire)
+  bool lmap = false;
+  uint32_t weight[32] = {};
 };
 
 static bool rot_enabled() {
@@ -1544,16 +1561,37 @@ static int run_sweep(mq_state* h, Sweep& sw, const std::vector<int>& op_phase, c
   for (size_t p = 0; p < sw.phases.size(); ++p) {
     const auto& regs = sw.phases[p];
     PhaseDesc& D = P.ph[p];
+    auto gword = [&](int b) { return sw.lmap ? sw.weight[sw.tile_bits[b]] : 1u << sw.tile_bits[b]; };
     for (int k = 0; k < lr; ++k) {
       D.s_reg[k] = phys(1u << regs[k]);
-      D.g_reg[k] = 1u << sw.tile_bits[regs[k]];
+      D.g_reg[k] = gword(regs[k]);
     }
-    int j = 0;
+    // thread bits: first those that spread the lanes of one shared-memory
+    // wavefront (16 of 8 bytes, 8 of 16) over its banks, then the rest in
+    // order.  Register bits on nibble boundaries leave the ascending order;
+    // scattered ones (a QFT's ordered wires) would put two lane bits on one bank
+    // bit, as index bits 1 and 4, 2 and 5 or 3 and 6 are
+    std::vector<int> grp, rest;
+    const bool wide = !c64 || regs[0] == 0;  // 16-byte accesses
+    const uint32_t banks = c64 ? 0xFu : 0x7u, skip = c64 && wide ? 1u : 0u;
+    uint32_t seen[4] = {};
     for (int b = 0; b < m; ++b) {
       if (std::find(regs.begin(), regs.end(), b) != regs.end()) continue;
-      D.s_grp[j] = phys(1u << b);
-      D.g_grp[j] = 1u << sw.tile_bits[b];
-      ++j;
+      uint32_t v = phys(1u << b) & banks & ~skip;
+      for (int i = 3; i >= 0; --i)
+        if ((v >> i) & 1u) {
+          if (!seen[i]) {
+            seen[i] = v;
+            break;
+          }
+          v ^= seen[i];
+        }
+      (v ? grp : rest).push_back(b);
+    }
+    grp.insert(grp.end(), rest.begin(), rest.end());
+    for (size_t j = 0; j < grp.size(); ++j) {
+      D.s_grp[j] = phys(1u << grp[j]);
+      D.g_grp[j] = gword(grp[j]);
     }
   }
   if (qft) {
@@ -1578,7 +1616,8 @@ static int run_sweep(mq_state* h, Sweep& sw, const std::vector<int>& op_phase, c
       int wmax = 0, gmin = 64, gmax = -1;
       for (int o = o0; o < o1 && chain; ++o) {
         const TileOp& op = P.ops[o];
-        const int g = sw.tile_bits[sw.phases[p][op.rk]];
+        const int gb = sw.tile_bits[sw.phases[p][op.rk]];
+        const int g = sw.lmap ? 31 - __builtin_clz(sw.weight[gb]) : gb;
         chain = op.lad_shift == P.ops[o0].lad_shift && op.width == g - (int)op.lad_shift;
         wmax = std::max(wmax, (int)op.width);
         gmin = std::min(gmin, g);
@@ -1653,6 +1692,19 @@ static int run_sweep(mq_state* h, Sweep& sw, const std::vector<int>& op_phase, c
     QftParams Q;
     std::memset(&Q, 0, sizeof(Q));
     static_cast<TileParams&>(Q) = P;
+    if (sw.lmap) {
+      Q.lmap = 1;
+      for (int i = 0; i < 4; ++i)
+        for (int x = 0; x < 256; ++x) {
+          const uint64_t t = (uint64_t)x << (8 * i);
+          if (t >= P.n_tiles) break;
+          const uint32_t b = deposit_runs((uint32_t)t, P.runs);
+          uint32_t v = 0;
+          for (int j = 0; j < h->n; ++j)
+            if ((b >> j) & 1u) v |= sw.weight[j];
+          Q.ltab[256 * i + x] = v;
+        }
+    }
     for (int w = 0; w < P.n_ops; ++w) {
       const TileOp& op = P.ops[w];
       const PhaseDesc& D = P.ph[op.phase];
@@ -2089,6 +2141,103 @@ int launch_qft_stages(mq_state* h, int q0, int k, int j_begin, int j_end, int in
       sw.ops.push_back(op);
     }
     // 2^{-cnt/2}: exact power of two for even counts
+    sw.scale = std::ldexp(1.0, -(cnt / 2)) * ((cnt & 1) ? 0.70710678118654752440 : 1.0);
+    sw.has_scale = true;
+    int rc = run_sweep(h, sw, op_phase, op_rk);
+    if (rc) return rc;
+  }
+  return MQ_OK;
+}
+
+// The same transform on any ordered wires (sim.py:522-563), without moving
+// them together: stage j acts on index bit bits[j], the ladder bits of its
+// phase are those of the later wires, wherever they are (QftParams::lmap).
+// The general tiles hold the low passengers beside a sweep's scattered
+// targets, so a sweep moves runs of 2^pas amplitudes as any high sweep does.
+// Before, the wires were permuted to the top of the register and back: 15 of
+// 25 qubits, inverse: four passes, 418 us; two sweeps, 226 us this way.
+int launch_qft_wires(mq_state* h, const int32_t* wires, int k, int inverse) {
+  const int n = h->n;
+  const int tmax = std::min(plan_tile_max(h), h->dtype == MQ_C64 ? 12 : 11);
+  const int pas = std::min(plan_passengers(h), n);
+  std::vector<int> bits(k);
+  Sweep proto;
+  proto.lmap = true;
+  for (int j = 0; j < k; ++j) {
+    bits[j] = n - 1 - wires[j];
+    proto.weight[bits[j]] = 1u << (k - 1 - j);
+  }
+  auto tile_of = [&](int j0, int cnt) {
+    std::vector<int> t;
+    for (int b = 0; b < std::max(pas, 1); ++b) t.push_back(b);
+    for (int j = j0; j < j0 + cnt; ++j)
+      if (bits[j] >= std::max(pas, 1)) t.push_back(bits[j]);
+    return t;
+  };
+  // as few groups of consecutive stages as fit their tiles, evenly filled
+  // where that fits too
+  auto split = [&](int most) {
+    std::vector<std::pair<int, int>> groups;
+    for (int j0 = 0; j0 < k;) {
+      int cnt = 1;
+      while (j0 + cnt < k && cnt < most && (int)tile_of(j0, cnt + 1).size() <= tmax) ++cnt;
+      groups.push_back({j0, cnt});
+      j0 += cnt;
+    }
+    return groups;
+  };
+  auto groups = split(kMaxOps);
+  const auto even = split((k + (int)groups.size() - 1) / (int)groups.size());
+  if (even.size() == groups.size()) groups = even;
+  if (inverse) std::reverse(groups.begin(), groups.end());
+  for (auto [j0, cnt] : groups) {
+    Sweep sw = proto;
+    sw.tile_bits = tile_of(j0, cnt);
+    // filled with low bits to 11 (complex64: 24 warps an SM where a 10-bit tile
+    // has 16; 113 against 120 us a sweep of 25 qubits, 12 bits 115; complex128:
+    // 92 against 105 us)
+    const int want = std::min({n, std::max(plan_min_tile(h), 11), tmax});
+    for (int b = 0; (int)sw.tile_bits.size() < want && b < n; ++b)
+      if (std::find(sw.tile_bits.begin(), sw.tile_bits.end(), b) == sw.tile_bits.end()) sw.tile_bits.push_back(b);
+    std::sort(sw.tile_bits.begin(), sw.tile_bits.end());
+    const int m = (int)sw.tile_bits.size();
+    if (m > tmax) return fail(MQ_EINVAL, "qft tile too large");
+    const int lr = reg_bits(h->dtype, m);
+    std::vector<int> stages;
+    for (int i = 0; i < cnt; ++i) stages.push_back(inverse ? j0 + cnt - 1 - i : j0 + i);
+    // register phases of lr stages; slots in the order of their ladder weight,
+    // bits that are no ladder bit of the phase's stages (other qubits, earlier
+    // wires) above them: a pair's factor reads the slots below its own
+    std::vector<int> op_phase(cnt), op_rk(cnt);
+    for (int i = 0; i < cnt; i += lr) {
+      std::vector<int> regs;
+      uint32_t top = 0;
+      for (int j = i; j < std::min(cnt, i + lr); ++j) {
+        regs.push_back(tile_local(sw.tile_bits, bits[stages[j]]));
+        top = std::max(top, sw.weight[bits[stages[j]]]);
+      }
+      auto key = [&](int b) {
+        const uint32_t w = sw.weight[sw.tile_bits[b]];
+        return w ? (uint64_t)w : (uint64_t(1) << 40) + (uint32_t)b;
+      };
+      for (int pass = 0; pass < 2; ++pass)  // padding above the stages first
+        for (int b = m - 1; (int)regs.size() < lr && b >= 0; --b)
+          if (std::find(regs.begin(), regs.end(), b) == regs.end() && (pass || key(b) > top)) regs.push_back(b);
+      std::sort(regs.begin(), regs.end(), [&](int a, int b) { return key(a) < key(b); });
+      for (int j = i; j < std::min(cnt, i + lr); ++j) {
+        op_phase[j] = (int)sw.phases.size();
+        op_rk[j] = (int)(std::find(regs.begin(), regs.end(), tile_local(sw.tile_bits, bits[stages[j]])) - regs.begin());
+      }
+      sw.phases.push_back(regs);
+    }
+    for (int i = 0; i < cnt; ++i) {
+      TileOp op;
+      std::memset(&op, 0, sizeof(op));
+      op.kind = inverse ? OP_QFT_INV : OP_QFT_FWD;
+      op.width = (uint8_t)(k - 1 - stages[i]);
+      if (op.width) sw.need_tw = true;
+      sw.ops.push_back(op);
+    }
     sw.scale = std::ldexp(1.0, -(cnt / 2)) * ((cnt & 1) ? 0.70710678118654752440 : 1.0);
     sw.has_scale = true;
     int rc = run_sweep(h, sw, op_phase, op_rk);
