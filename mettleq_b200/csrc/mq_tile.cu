@@ -129,6 +129,9 @@ constexpr int kEpiLutBytes = 16384;
 // (narrower windows, one more lookup per 16-amplitude group), which keeps
 // the sweep at the occupancy of a plain one.
 constexpr int kRegDiagSmall = 1024;
+// complex128: 320 entries (5 KB) beside the two 32 KB tiles keep three CTAs on
+// an SM; with 1024 entries the low sweep of a 25-qubit layer ran two (314 us, 276 us with three)
+constexpr int reg_diag_small(int dtype) { return dtype == MQ_C64 ? kRegDiagSmall : 320; }
 // A diagonal applied to a 4-bit register phase: windows [0, n_win) taken at
 // the group base, times T[c][r] at lut[toff + 17c + r] (c = index bits
 // cbit[0..nc); rows padded to 17 entries against bank conflicts).
@@ -965,22 +968,25 @@ k_tile(const V2<R>* src, V2<R>* dst, const __grid_constant__ PT P) {
         }
       }
     }
-    if constexpr (STORE_EPI && TMA && CB == 1) {
+    if constexpr (STORE_EPI && TMA) {
       if (P.tma.store == 2) {
-        // permutation keeping index bit 0: output chunk c = tid + k*NT is the
-        // input pair at l0 = cl ^ A(c << 1) (swapped when l0 is odd).  Every
-        // thread reads its chunks, the barrier ends all reads of the tile,
-        // the chunks go to their output slots, and the tile leaves as one
-        // TMA store to output tile `tile`
+        // output chunk c = tid + k*NT is the input chunk at l0 = cl ^ A(c << CB):
+        // one complex128 amplitude, or the complex64 pair of a permutation
+        // keeping index bit 0 (swapped when l0 is odd).  Every thread reads
+        // its chunks, the barrier ends all reads of the tile, the chunks go
+        // to their output slots, and the tile leaves as one TMA store to
+        // output tile `tile`.  complex128, 25 qubits: 314 us for the low
+        // sweep against 364 us with per-thread stores
+        float4* c4w = reinterpret_cast<float4*>(cur);
         float4 v[CPT];
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
           const uint32_t l0 = cl_in ^ epi_at ^ chunk_cols<LT, LCH, CB>(k, ecols);
-          const float4 w = *reinterpret_cast<const float4*>(cur + amp_slot<R>(l0 & ~1u));
-          v[k] = (l0 & 1u) ? make_float4(w.z, w.w, w.x, w.y) : w;
+          const uint32_t ch = l0 >> CB;
+          const float4 w = c4w[ch ^ ((ch >> 3) & 7u)];
+          v[k] = (CB == 1 && (l0 & 1u)) ? make_float4(w.z, w.w, w.x, w.y) : w;
         }
         __syncthreads();
-        float4* c4w = reinterpret_cast<float4*>(cur);
 #pragma unroll
         for (int k = 0; k < CPT; ++k) c4w[slot(k)] = v[k];
         fence_proxy_async_smem();
@@ -1534,13 +1540,13 @@ static int run_sweep(mq_state* h, Sweep& sw, const std::vector<int>& op_phase, c
   for (int k = 0; k < m; ++k) P.tile_bit[k] = (uint8_t)sw.tile_bits[k];
   make_base_runs(P.runs, h->n, P.tile_bit, m);
   // TMA form for tiles of 10 bits and more whose shape it can describe.
-  // Write-back: a TMA store of the tile in place (1); for a permutation that
-  // keeps index bit 0 (complex64, no window diagonal), the output tile is
-  // gathered in shared memory and then TMA-stored (2); otherwise per-thread
-  // stores (0)
+  // Write-back: a TMA store of the tile in place (1); for a permutation
+  // (complex64: one that keeps index bit 0) without a window diagonal, the
+  // output tile is gathered in shared memory and then TMA-stored (2);
+  // otherwise per-thread stores (0)
   if (tma_enabled() && m >= 10 && !sw.phases.empty() && plan_tma(h->n, h->amp_bytes(), sw.tile_bits, P.tma)) {
     if (!epi || (!epi->perm && !epi->diag)) P.tma.store = 1;
-    else if (epi->perm && !epi->diag && epi->cols[0] == 1u && h->dtype == MQ_C64 && tma_perm_store()) P.tma.store = 2;
+    else if (epi->perm && !epi->diag && (h->dtype == MQ_C128 || epi->cols[0] == 1u) && tma_perm_store()) P.tma.store = 2;
     else P.tma.store = 0;
   }
   // chunk-index bits above the thread bits: contiguous global bits?
@@ -1916,7 +1922,7 @@ static int launch_layer_euler(mq_state* h, const double* mats, int n_terms, cons
     const auto& regs = low.phases.back();
     const int rb[4] = {regs[0], regs[1], regs[2], regs[3]};
     // small tables first: they share the SM's shared memory with the tile
-    for (int budget : {kRegDiagSmall, max_entries}) {
+    for (int budget : {reg_diag_small(h->dtype), max_entries}) {
       int rc = plan_diag_register(h, (int)post_k.size(), post_k.data(), post_w.data(), post_p.data(), rb, budget,
                                   e.reg);
       if (rc) return rc;
@@ -1947,7 +1953,7 @@ static int launch_layer_euler(mq_state* h, const double* mats, int n_terms, cons
     for (int k = 0; k < 4; ++k) rb[k] = fs.tile_bits[fs.phases.front()[k]];
     DiagRegister& pr = has_high ? e_first.pre_reg : e.pre_reg;
     const int room = has_high ? max_entries : max_entries - (int)(e.reg.win.vals.size() / 2);
-    for (int budget : {std::min(room, kRegDiagSmall / 2), room}) {
+    for (int budget : {std::min(room, h->dtype == MQ_C64 ? kRegDiagSmall / 2 : reg_diag_small(MQ_C128)), room}) {
       int rc = plan_diag_register(h, (int)pre_k.size(), pre_k.data(), pre_w.data(), pre_p.data(), rb, budget, pr);
       if (rc) return rc;
       if (pr.win.n >= 0) break;
@@ -2033,7 +2039,7 @@ int launch_layer(mq_state* h, const double* mats, const uint8_t* active, int n_t
     if (low_u2 && !low.phases.empty() && low.phases.back().size() == 4 && m >= 4) {
       const auto& regs = low.phases.back();
       const int rb[4] = {regs[0], regs[1], regs[2], regs[3]};
-      for (int budget : {kRegDiagSmall, max_entries}) {
+      for (int budget : {reg_diag_small(h->dtype), max_entries}) {
         int rc = plan_diag_register(h, n_terms, kinds, wires, params, rb, budget, e.reg);
         if (rc) return rc;
         if (e.reg.win.n >= 0) break;
