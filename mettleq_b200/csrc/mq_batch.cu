@@ -11,10 +11,10 @@
 //     atomic counter, start from |0...0>, apply every layer in place (the
 //     ladder is a gather between two shared buffers) and write the
 //     probabilities and <Z_0>; nothing but the outputs touches HBM;
-//   * larger circuits run the fused-layer tile sweeps on per-lane states
-//     (one stream per lane, the lanes are parallel branches of the graph, so
-//     small sweeps of different circuits overlap on the device), followed by
-//     k_probs_z.
+//   * larger circuits run in groups of one width (k_group_sweep), one launch
+//     per layer and sweep for the whole group, on parallel lanes (one stream
+//     each, the lanes are parallel branches of the graph).  With a tile plan of
+//     mq_batch_set_tiles they run one by one through the general tile sweeps.
 //
 // Gate matrices live in device memory (read by the kernels when they run),
 // so one captured graph serves every later parameter set: a run is one
@@ -136,6 +136,326 @@ __global__ void __launch_bounds__(NT) k_batch_small(const SmallCircuit* __restri
   }
 }
 
+// ------------------------------------------------- groups of larger circuits
+// Circuits of one width (and ladder choice) run together, sorted by depth:
+// their states lie one after the other, and a layer of all circuits that are
+// still that deep is one launch per sweep.  A sweep of one 14- to 20-qubit
+// circuit fills a fraction of the GPU for about 10 us, and a graph of one such
+// node per circuit, layer and sweep is bound by its nodes: 256 circuits of 10
+// to 20 qubits, 9.0 ms with 3400 sweeps of single circuits, 4.7 ms this way (20
+// qubits, 32 circuits: 5.2 -> 3.5 ms; 14 and 15 qubits, 100 circuits: 1.54 -> 0.42).
+// What bounds a sweep now is the complex 2x2 arithmetic and its latency (24 warps
+// an SM).  The gates of an amplitude are applied in the order and with the
+// rounding of the single circuits' sweeps (fill_order): the states are the same
+// bits.
+struct GroupCirc {
+  uint64_t mats_off;   // doubles: the circuit's matrices, layer-major
+  uint64_t probs_off;  // floats
+  uint32_t index, depth;
+};
+
+struct GroupSweep {
+  const float2* src;
+  float2* dst;
+  const GroupCirc* circ;
+  const double* mats;
+  uint32_t layer;
+  uint32_t n_tiles;    // circuits << (n - 12)
+  uint8_t n, start, cnt;  // target bits [start, start + cnt)
+  uint8_t ladder;      // low sweep: CNOT ladder at the write-back
+};
+
+// Tile-local index of register pattern r of the thread's group, register bits
+// [4P, 4P + 4).
+template <int P>
+__device__ __forceinline__ uint32_t nib_index(uint32_t tid, uint32_t r) {
+  if constexpr (P == 0) return (tid << 4) | r;
+  else if constexpr (P == 1) return (tid & 15u) | (r << 4) | ((tid >> 4) << 8);
+  else return tid | (r << 8);
+}
+
+constexpr int kSweepThreads = 256;
+constexpr int kSweepCtas = 3;  // 80 registers a thread: 4.68 ms a batch run; 4.90 with 2 CTAs, 5.51 with 4
+
+// One phase: 16 amplitudes differing in tile bits [4P, 4P + 4), the gates of
+// the first `cnt` of these bits in ascending order.  um: every matrix entry u
+// as the pairs (u.x, u.x), (-u.y, u.y), so that a component pair of cmac2f is
+// four paired FP32 instructions in its order (the same roundings): 5.19 -> 4.98
+// ms a batch run.
+template <int P>
+__device__ __forceinline__ void group_phase(float2* tile, uint32_t tid, int cnt, const float4 (*um)[4]) {
+  float2 a[16];
+  if constexpr (P == 0) {
+#pragma unroll
+    for (int r = 0; r < 16; r += 2) {
+      const float4 v = *reinterpret_cast<const float4*>(tile + bslot(nib_index<P>(tid, r)));
+      a[r] = make_float2(v.x, v.y);
+      a[r + 1] = make_float2(v.z, v.w);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < 16; ++r) a[r] = tile[bslot(nib_index<P>(tid, r))];
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k >= cnt) break;
+    float2 u[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 q = um[k][j];
+      u[j][0] = make_float2(q.x, q.y);
+      u[j][1] = make_float2(q.z, q.w);
+    }
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      if (r & (1 << k)) continue;
+      const float2 x0 = a[r], x1 = a[r | (1 << k)];
+      const float2 s0 = make_float2(x0.y, x0.x), s1 = make_float2(x1.y, x1.x);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        a[j ? (r | (1 << k)) : r] =
+            __ffma2_rn(x0, u[2 * j][0],
+                       __ffma2_rn(s0, u[2 * j][1], __ffma2_rn(x1, u[2 * j + 1][0], __fmul2_rn(s1, u[2 * j + 1][1]))));
+    }
+  }
+  if constexpr (P == 0) {
+#pragma unroll
+    for (int r = 0; r < 16; r += 2)
+      *reinterpret_cast<float4*>(tile + bslot(nib_index<P>(tid, r))) =
+          make_float4(a[r].x, a[r].y, a[r + 1].x, a[r + 1].y);
+  } else {
+#pragma unroll
+    for (int r = 0; r < 16; ++r) tile[bslot(nib_index<P>(tid, r))] = a[r];
+  }
+}
+
+// A sweep of one layer over a group: tiles of 2^12 amplitudes, register phases
+// on the tile's nibbles, from the top target bits down.  LOW: the tile is the
+// index bits [0, 12), targets [0, cnt), the ladder out[y] = in[y ^ (y >> 1)] at
+// the write-back (an output tile reads one input tile).  Else cnt <= 8 high
+// targets in tile bits [4, 4 + cnt) over the passengers 0-3; the tile's
+// remaining bits are the index bits from 4 up, so a run is 2^(12 - cnt)
+// amplitudes.  In place unless the ladder permutes.
+template <bool LOW>
+__global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_group_sweep(const __grid_constant__ GroupSweep P) {
+  __shared__ __align__(16) float2 tile[4096];
+  __shared__ float4 um[12][4];  // by tile bit
+  uint32_t tid = threadIdx.x;
+  const int n = P.n, cnt = P.cnt, pas = 12 - cnt;
+  uint32_t have = 0xffffffffu;
+  for (uint32_t t = blockIdx.x; t < P.n_tiles; t += gridDim.x) {
+    // keeps the per-chunk addresses from being held (spilled) across tiles
+    asm volatile("" : "+r"(tid));
+    const uint32_t cid = t >> (n - 12);
+    const uint32_t h = t & ((1u << (n - 12)) - 1u);
+    const size_t state = (size_t)cid << n;
+    uint32_t base;  // of the input tile
+    if constexpr (LOW) {
+      base = (P.ladder ? h ^ (h >> 1) : h) << 12;
+    } else {
+      const int run = P.start - pas;  // free bits between the passengers and the targets
+      base = ((h & ((1u << run) - 1u)) << pas) | ((h >> run) << (P.start + cnt));
+    }
+    // consecutive chunks of a tile are consecutive in memory: chunk order over
+    // (passengers, targets), tile-local order (passengers 0-3, targets, other
+    // passengers)
+    auto local_of = [&](uint32_t i) -> uint32_t {
+      if constexpr (LOW) return i;
+      const uint32_t low = i & 15u, mid = (i >> 4) & ((1u << (pas - 4)) - 1u), tg = i >> pas;
+      return low | (tg << 4) | (mid << (4 + cnt));
+    };
+    auto global_of = [&](uint32_t i) -> uint32_t {
+      if constexpr (LOW) return base | i;
+      else return base | (i & ((1u << pas) - 1u)) | ((i >> pas) << P.start);
+    };
+    __syncthreads();  // the previous tile has left
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t i = 2 * tid + 512 * k;
+      cp_async<16>(smem_u32(tile + bslot(local_of(i))), P.src + state + global_of(i));
+    }
+    cp_async_commit();
+    if (cid != have) {
+      have = cid;
+      if ((int)tid < 4 * cnt) {
+        const int j = tid >> 2;
+        const double* m = P.mats + P.circ[cid].mats_off + ((size_t)P.layer * n + (n - 1 - (P.start + j))) * 8;
+        const float x = (float)m[2 * (tid & 3u)], y = (float)m[2 * (tid & 3u) + 1];
+        um[(LOW ? 0 : 4) + j][tid & 3u] = make_float4(x, x, -y, y);
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if constexpr (LOW) {
+      if (cnt > 8) {
+        group_phase<2>(tile, tid, cnt - 8, &um[8]);
+        __syncthreads();
+      }
+      if (cnt > 4) {
+        group_phase<1>(tile, tid, min(cnt - 4, 4), &um[4]);
+        __syncthreads();
+      }
+      group_phase<0>(tile, tid, min(cnt, 4), &um[0]);
+    } else {
+      if (cnt > 4) {
+        group_phase<2>(tile, tid, cnt - 4, &um[8]);
+        __syncthreads();
+      }
+      group_phase<1>(tile, tid, min(cnt, 4), &um[4]);
+    }
+    __syncthreads();
+    float2* out = P.dst + state;
+    const uint32_t cl = (h & 1u) << 11;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t i = 2 * tid + 512 * k;
+      if constexpr (LOW) {
+        uint32_t l = i;
+        if (P.ladder) l = i ^ (i >> 1) ^ cl;
+        const float4 v = *reinterpret_cast<const float4*>(tile + bslot(l & ~1u));
+        *reinterpret_cast<float4*>(out + ((h << 12) | i)) = (l & 1u) ? make_float4(v.z, v.w, v.x, v.y) : v;
+      } else {
+        *reinterpret_cast<float4*>(out + global_of(i)) = *reinterpret_cast<const float4*>(tile + bslot(local_of(i)));
+      }
+    }
+  }
+}
+
+// The state after the first layer, written once instead of a cleared state and
+// a layer of sweeps on it: from |0...0> every amplitude is the product of one
+// entry of each qubit's first column, multiplied up in the order of the
+// sweeps' gates (then the ladder).  Circuits without layers stay |0...0>.
+struct GroupFirst {
+  float2* dst;
+  const GroupCirc* circ;
+  const double* mats;
+  uint32_t n_tiles;
+  uint8_t n, ladder;
+  uint8_t order[32];  // index bits in gate order; the last four are 0, 1, 2, 3
+};
+__global__ void __launch_bounds__(kSweepThreads) k_group_first(const __grid_constant__ GroupFirst P) {
+  __shared__ float2 col[32][2];  // by gate order
+  const uint32_t tid = threadIdx.x;
+  const int n = P.n;
+  // a gate on amplitudes (v, 0): the rounding of cmac2f with x1 = 0
+  auto times = [](float2 u, float2 v) { return make_float2(fmaf(u.x, v.x, -u.y * v.y), fmaf(u.x, v.y, u.y * v.x)); };
+  uint32_t have = 0xffffffffu;
+  for (uint32_t t = blockIdx.x; t < P.n_tiles; t += gridDim.x) {
+    const uint32_t cid = t >> (n - 12);
+    const uint32_t h = t & ((1u << (n - 12)) - 1u);
+    const uint32_t depth = P.circ[cid].depth;
+    if (cid != have) {
+      have = cid;
+      __syncthreads();
+      if ((int)tid < 2 * n) {
+        const int j = tid >> 1, e = tid & 1;
+        float2 v = make_float2(e ? 0.f : 1.f, 0.f);
+        if (depth) {
+          const double* m = P.mats + P.circ[cid].mats_off + (size_t)(n - 1 - P.order[j]) * 8 + 4 * e;
+          v = make_float2((float)m[0], (float)m[1]);
+        }
+        col[j][e] = v;
+      }
+      __syncthreads();
+    }
+    const bool lad = P.ladder && depth;
+    float2* out = P.dst + ((size_t)cid << n);
+    // 16 amplitudes of the product, consecutive before the ladder: the ladder
+    // maps them to 16 of one 16-aligned run of outputs
+    const uint32_t x0 = ((lad ? h ^ (h >> 1) : h) << 12) | (tid << 4);
+    // (the low 12 bits are enumerated over all threads, so the tile's set of
+    // inputs is the set its outputs read)
+    float2 v[16];
+    v[0] = make_float2(1.f, 0.f);
+    for (int j = 0; j < n - 4; ++j) v[0] = times(col[j][(x0 >> P.order[j]) & 1u], v[0]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 c0 = col[n - 4 + k][0], c1 = col[n - 4 + k][1];
+#pragma unroll
+      for (int r = 0; r < (1 << k); ++r) {
+        v[r | (1 << k)] = times(c1, v[r]);
+        v[r] = times(c0, v[r]);
+      }
+    }
+    // output index of input x: y ^ (y >> 1) = x, the prefix XOR from the top;
+    // the low 12 bits start from the parity of the bits above
+    uint32_t y0 = x0 & 4095u;
+    if (lad) {
+      y0 ^= y0 >> 1;
+      y0 ^= y0 >> 2;
+      y0 ^= y0 >> 4;
+      y0 ^= y0 >> 8;
+      y0 &= 4095u;
+      if (h & 1u) y0 ^= 4095u;  // y's bit 12 is h's bit 0
+    }
+    const uint32_t at = (h << 12) | (y0 & ~15u);
+    const uint32_t top = (y0 & 16u) ? 15u : 0u;  // y's bit 4 flips the prefix of the low four
+#pragma unroll
+    for (int r = 0; r < 16; r += 2) {
+      // outputs (e, e + 1) of the run, e even, read inputs g(e), g(e) ^ 1
+      const int g = r ^ (r >> 1);
+      if (lad) {
+        const uint32_t e = (uint32_t)r ^ top;  // output offset whose input pattern is g(r), or its partner
+        const float2 p = v[g & 15], q = v[(g ^ 1) & 15];
+        // e and e ^ 1 are one pair; e is odd when top is set
+        *reinterpret_cast<float4*>(out + at + (e & ~1u)) =
+            (e & 1u) ? make_float4(q.x, q.y, p.x, p.y) : make_float4(p.x, p.y, q.x, q.y);
+      } else {
+        *reinterpret_cast<float4*>(out + at + r) = make_float4(v[r].x, v[r].y, v[r + 1].x, v[r + 1].y);
+      }
+    }
+  }
+}
+
+// Probabilities and per-block partial sums of <Z_0> of a group: `blocks`
+// blocks per circuit; a circuit's state is in the buffer its number of
+// permuted layers left it in.
+struct GroupProbs {
+  const float2* buf[2];
+  const GroupCirc* circ;
+  float* probs;
+  double* zpart;
+  uint32_t blocks;
+  uint8_t n, ladder;
+};
+__global__ void __launch_bounds__(256) k_group_probs(const __grid_constant__ GroupProbs P) {
+  __shared__ double red[8];
+  const uint32_t cid = blockIdx.x / P.blocks, block = blockIdx.x % P.blocks;
+  const GroupCirc C = P.circ[cid];
+  const float2* st = P.buf[(P.ladder && C.depth > 1) ? ((C.depth - 1) & 1u) : 0u] + ((size_t)cid << P.n);
+  float* probs = P.probs + C.probs_off;
+  const uint32_t pairs = 1u << (P.n - 1);
+  double acc = 0.0;
+  for (uint32_t i = block * 256u + threadIdx.x; i < pairs; i += P.blocks * 256u) {
+    const float4 v = reinterpret_cast<const float4*>(st)[i];
+    const double p0 = (double)v.x * v.x + (double)v.y * v.y, p1 = (double)v.z * v.z + (double)v.w * v.w;
+    probs[2 * i] = (float)p0;
+    probs[2 * i + 1] = (float)p1;
+    acc += ((i >> (P.n - 2)) & 1u) ? -(p0 + p1) : p0 + p1;
+  }
+#pragma unroll
+  for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double z = 0.0;
+    for (int w = 0; w < 8; ++w) z += red[w];
+    P.zpart[blockIdx.x] = z;
+  }
+}
+// <Z_0> of the group's circuits from their blocks' sums, a warp each
+__global__ void k_group_z(const double* __restrict__ zpart, uint32_t blocks, const GroupCirc* __restrict__ circ,
+                          uint32_t count, double* __restrict__ z0) {
+  const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= count) return;
+  const uint32_t lane = threadIdx.x & 31;
+  double z = 0.0;
+  for (uint32_t b = lane; b < blocks; b += 32) z += zpart[(size_t)c * blocks + b];
+#pragma unroll
+  for (int off = 16; off; off >>= 1) z += __shfl_xor_sync(0xffffffffu, z, off);
+  if (lane == 0) z0[circ[c].index] = z;
+}
+
 // probabilities of a full state and per-block partial sums of <Z_0>
 __global__ void __launch_bounds__(256) k_probs_z(const float2* __restrict__ st, uint32_t dim, int n,
                                                  float* __restrict__ probs, double* __restrict__ zpart) {
@@ -192,13 +512,25 @@ struct mq_batch {
   // large circuits
   std::vector<int> large;
   int lanes = 1;
-  std::vector<std::vector<int>> lane_work;
+  std::vector<std::vector<int>> lane_work;  // single circuits (plan_singles)
+  // groups of circuits of one width and ladder choice, deepest first
+  struct Group {
+    int n = 0;
+    bool ladder = false;
+    std::vector<int> circ;
+    uint32_t first = 0;  // their GroupCirc entries start here
+  };
+  std::vector<Group> groups;
+  std::vector<std::vector<int>> lane_groups;
+  std::vector<float2*> lane_buf[2];
+  GroupCirc* d_group = nullptr;
   std::vector<cudaStream_t> lane_stream;
   std::vector<cudaEvent_t> lane_event;
   cudaEvent_t fork_event = nullptr;
   std::vector<std::map<int, mq_state*>> lane_state;
   double* d_zpart = nullptr;
-  uint32_t zblocks = 0;
+  uint32_t zblocks = 0;   // most blocks of one circuit
+  size_t zslots = 0;      // partial sums of a lane
   int num_sms = 148;
   // sweep plan of the large circuits (mq_batch_set_tiles; 0 / -1 = defaults)
   int tile_max = 0, tile_pas = -1, tile_min = 0;
@@ -227,6 +559,10 @@ static void batch_free(mq_batch* b) {
   if (b->d_small) cudaFree(b->d_small);
   if (b->d_next) cudaFree(b->d_next);
   if (b->d_zpart) cudaFree(b->d_zpart);
+  for (auto& v : b->lane_buf)
+    for (float2* p : v)
+      if (p) cudaFree(p);
+  if (b->d_group) cudaFree(b->d_group);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }
@@ -282,47 +618,255 @@ static int small_dispatch(mq_batch* b, float* probs, double* z0, bool configure)
   }
 }
 
+// The large circuits of a lane one by one through the general sweeps, with the
+// tile plan of mq_batch_set_tiles.
+static int record_lane_single(mq_batch* b, int l, float* probs, double* z0) {
+  uint32_t cols[32];
+  cudaStream_t s = b->lane_stream[l];
+  double* zpart = b->d_zpart + (size_t)l * b->zslots;
+  for (int c : b->lane_work[l]) {
+    const int n = b->n[c];
+    mq_state* h = nullptr;
+    int rc = lane_state_for(b, l, n, &h);
+    if (rc) return rc;
+    h->cur = 0;
+    MQ_CUDA(cudaMemsetAsync(h->buf[0], 0, h->state_bytes, s));
+    k_basis0<<<1, 32, 0, s>>>(reinterpret_cast<float2*>(h->buf[0]));
+    MQ_LAUNCHED("k_basis0");
+    // CNOT ladder: columns A e_j of out[y] = in[A y], A e_j = e_j + e_{j-1}
+    for (int j = 0; j < n; ++j) cols[j] = (1u << j) | (j ? (1u << (j - 1)) : 0u);
+    for (int d = 0; d < b->depth[c]; ++d) {
+      const double* md = b->d_mats + b->mats_off[c] + (size_t)d * n * 8;
+      rc = launch_layer(h, nullptr, nullptr, 0, nullptr, nullptr, nullptr, b->ladder[c] ? cols : nullptr, 0, md);
+      if (rc) return rc;
+    }
+    const uint32_t dim = 1u << n;
+    const uint32_t grid = std::min<uint32_t>(b->zblocks, std::max<uint32_t>(1, dim / 256));
+    k_probs_z<<<grid, 256, 0, s>>>(reinterpret_cast<const float2*>(h->cur_buf()), dim, n, probs + b->probs_off[c], zpart);
+    MQ_LAUNCHED("k_probs_z");
+    k_zsum<<<1, 32, 0, s>>>(zpart, grid, z0 + c);
+    MQ_LAUNCHED("k_zsum");
+  }
+  return MQ_OK;
+}
+
+// <Z_0> blocks of one circuit of a group: 16 pairs of amplitudes a thread,
+// at most zblocks.
+static uint32_t group_blocks(const mq_batch* b, int n) {
+  return (uint32_t)std::min<uint64_t>(b->zblocks, std::max<uint64_t>(1, (uint64_t(1) << n) / 8192));
+}
+
+// Target bits (start, count) of a layer's sweeps on n qubits, the low sweep
+// first in the list and last in the layer: the split of the general sweeps
+// with 12-bit tiles and four passengers (mq_tile.cu split_bits).
+static std::vector<std::pair<int, int>> group_split(int n) {
+  const int n_hi = (n - 12 + 7) / 8;
+  const int low = std::max(n - n_hi * 8, std::min(12, (n + n_hi) / (n_hi + 1)));
+  std::vector<std::pair<int, int>> out = {{0, low}};
+  int start = low;
+  for (int i = 0; i < n_hi; ++i) {
+    const int cnt = (n - low) / n_hi + (i < (n - low) % n_hi ? 1 : 0);
+    out.push_back({start, cnt});
+    start += cnt;
+  }
+  return out;
+}
+// The index bits in the order their gates are applied to an amplitude: the
+// high sweeps, then the low one; in a sweep the remainder of its bits over
+// four from the top, then nibbles downwards, each ascending.
+static void fill_order(const std::vector<std::pair<int, int>>& split, uint8_t* order) {
+  int k = 0;
+  for (size_t i = 1; i <= split.size(); ++i) {
+    const auto [start, cnt] = split[i % split.size()];
+    for (int at = start + cnt; at > start;) {
+      const int len = (at - start) % 4 ? (at - start) % 4 : 4;
+      at -= len;
+      for (int b = 0; b < len; ++b) order[k++] = (uint8_t)(at + b);
+    }
+  }
+}
+
+static int record_lane_groups(mq_batch* b, int l, float* probs, double* z0) {
+  cudaStream_t s = b->lane_stream[l];
+  double* zpart = b->d_zpart + (size_t)l * b->zslots;
+  float2* buf[2] = {b->lane_buf[0][l], b->lane_buf[1][l]};
+  for (int gi : b->lane_groups[l]) {
+    const mq_batch::Group& G = b->groups[gi];
+    const int n = G.n;
+    const uint32_t count = (uint32_t)G.circ.size();
+    auto grid = [&](uint32_t tiles) { return std::min<uint32_t>(tiles, (uint32_t)b->num_sms * kSweepCtas); };
+    const auto split = group_split(n);
+    GroupFirst F;
+    std::memset(&F, 0, sizeof(F));
+    F.dst = buf[0];
+    F.circ = b->d_group + G.first;
+    F.mats = b->d_mats;
+    F.n_tiles = count << (n - 12);
+    F.n = (uint8_t)n;
+    F.ladder = G.ladder;
+    fill_order(split, F.order);
+    k_group_first<<<grid(F.n_tiles), kSweepThreads, 0, s>>>(F);
+    MQ_LAUNCHED("k_group_first");
+    int cur = 0;
+    for (int d = 1; d < b->depth[G.circ[0]]; ++d) {
+      uint32_t live = 0;
+      while (live < count && b->depth[G.circ[live]] > d) ++live;
+      GroupSweep P;
+      std::memset(&P, 0, sizeof(P));
+      P.circ = b->d_group + G.first;
+      P.mats = b->d_mats;
+      P.layer = (uint32_t)d;
+      P.n_tiles = live << (n - 12);
+      P.n = (uint8_t)n;
+      P.ladder = G.ladder;
+      P.src = P.dst = buf[cur];
+      for (size_t g = 1; g < split.size(); ++g) {
+        P.start = (uint8_t)split[g].first;
+        P.cnt = (uint8_t)split[g].second;
+        k_group_sweep<false><<<grid(P.n_tiles), kSweepThreads, 0, s>>>(P);
+        MQ_LAUNCHED("k_group_sweep");
+      }
+      if (G.ladder) cur ^= 1;
+      P.dst = buf[cur];
+      P.start = 0;
+      P.cnt = (uint8_t)split[0].second;
+      k_group_sweep<true><<<grid(P.n_tiles), kSweepThreads, 0, s>>>(P);
+      MQ_LAUNCHED("k_group_sweep");
+    }
+    GroupProbs Q;
+    Q.buf[0] = buf[0];
+    Q.buf[1] = buf[1];
+    Q.circ = b->d_group + G.first;
+    Q.probs = probs;
+    Q.zpart = zpart;
+    Q.blocks = group_blocks(b, n);
+    Q.n = (uint8_t)n;
+    Q.ladder = G.ladder;
+    k_group_probs<<<count * Q.blocks, 256, 0, s>>>(Q);
+    MQ_LAUNCHED("k_group_probs");
+    k_group_z<<<(count + 3) / 4, 128, 0, s>>>(zpart, Q.blocks, Q.circ, count, z0);
+    MQ_LAUNCHED("k_group_z");
+  }
+  return MQ_OK;
+}
+
+static bool single_circuits(const mq_batch* b) { return b->tile_max != 0 || b->tile_pas >= 0 || b->tile_min != 0; }
+
 // Record the whole batch on b->stream (being captured).
 static int record_batch(mq_batch* b, float* probs, double* z0) {
+  const bool single = single_circuits(b);
+  if (!b->large.empty()) {
+    MQ_CUDA(cudaEventRecord(b->fork_event, b->stream));
+    for (int l = 0; l < b->lanes; ++l) MQ_CUDA(cudaStreamWaitEvent(b->lane_stream[l], b->fork_event, 0));
+  }
   if (!b->small.empty()) {
     MQ_CUDA(cudaMemsetAsync(b->d_next, 0, sizeof(uint32_t), b->stream));
     int rc = small_dispatch(b, probs, z0, false);
     if (rc) return rc;
   }
   if (b->large.empty()) return MQ_OK;
-  MQ_CUDA(cudaEventRecord(b->fork_event, b->stream));
-  for (int l = 0; l < b->lanes; ++l) MQ_CUDA(cudaStreamWaitEvent(b->lane_stream[l], b->fork_event, 0));
-  uint32_t cols[32];
   for (int l = 0; l < b->lanes; ++l) {
-    cudaStream_t s = b->lane_stream[l];
-    double* zpart = b->d_zpart + (size_t)l * b->zblocks;
-    for (int c : b->lane_work[l]) {
-      const int n = b->n[c];
-      mq_state* h = nullptr;
-      int rc = lane_state_for(b, l, n, &h);
-      if (rc) return rc;
-      h->cur = 0;
-      MQ_CUDA(cudaMemsetAsync(h->buf[0], 0, h->state_bytes, s));
-      k_basis0<<<1, 32, 0, s>>>(reinterpret_cast<float2*>(h->buf[0]));
-      MQ_LAUNCHED("k_basis0");
-      // CNOT ladder: columns A e_j of out[y] = in[A y], A e_j = e_j + e_{j-1}
-      for (int j = 0; j < n; ++j) cols[j] = (1u << j) | (j ? (1u << (j - 1)) : 0u);
-      for (int d = 0; d < b->depth[c]; ++d) {
-        const double* md = b->d_mats + b->mats_off[c] + (size_t)d * n * 8;
-        rc = launch_layer(h, nullptr, nullptr, 0, nullptr, nullptr, nullptr, b->ladder[c] ? cols : nullptr, 0, md);
-        if (rc) return rc;
-      }
-      const uint32_t dim = 1u << n;
-      const uint32_t grid = std::min<uint32_t>(b->zblocks, std::max<uint32_t>(1, dim / 256));
-      k_probs_z<<<grid, 256, 0, s>>>(reinterpret_cast<const float2*>(h->cur_buf()), dim, n, probs + b->probs_off[c], zpart);
-      MQ_LAUNCHED("k_probs_z");
-      k_zsum<<<1, 32, 0, s>>>(zpart, grid, z0 + c);
-      MQ_LAUNCHED("k_zsum");
-    }
-    MQ_CUDA(cudaEventRecord(b->lane_event[l], s));
+    int rc = single ? MQ_OK : record_lane_groups(b, l, probs, z0);
+    if (!rc) rc = record_lane_single(b, l, probs, z0);
+    if (rc) return rc;
+    MQ_CUDA(cudaEventRecord(b->lane_event[l], b->lane_stream[l]));
     MQ_CUDA(cudaStreamWaitEvent(b->stream, b->lane_event[l], 0));
   }
   return MQ_OK;
+}
+
+// Most amplitudes of a group (32 MB; a wider circuit is a group of its own).
+// 256 circuits of 10 to 20 qubits on 16 lanes: 4.91 ms a run with 2^20, 4.79 with
+// 2^21, 4.68 with 2^22, 4.80 with 2^23.
+constexpr size_t kGroupAmps = size_t(1) << 22;
+
+
+// The large circuits that run one by one, all of them with a tile plan set by
+// mq_batch_set_tiles, else those of 24 qubits and more, where the general
+// sweeps with TMA tiles are as fast (24 qubits, 6
+// circuits: 12.5 ms both; 23 qubits, 8: 8.6 against 8.2 ms in groups): their
+// lanes (longest processing time
+// first) and the lanes' states, with the tile plan set so far.
+constexpr int kGroupMaxQubits = 23;
+static int plan_singles(mq_batch* b) {
+  for (auto& m : b->lane_state)
+    for (auto& kv : m) {
+      kv.second->tile_max = b->tile_max;
+      kv.second->tile_pas = b->tile_pas;
+      kv.second->tile_min = b->tile_min;
+    }
+  b->lane_work.assign(b->lanes, {});
+  b->lane_state.resize(b->lanes);
+  std::vector<int> order;
+  for (int c : b->large)
+    if (single_circuits(b) || b->n[c] > kGroupMaxQubits) order.push_back(c);
+  auto load = [&](int c) { return (uint64_t)std::max(1, b->depth[c]) << b->n[c]; };
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return load(x) > load(y); });
+  std::vector<uint64_t> sum(b->lanes, 0);
+  for (int c : order) {
+    const int l = (int)(std::min_element(sum.begin(), sum.end()) - sum.begin());
+    b->lane_work[l].push_back(c);
+    sum[l] += load(c);
+    mq_state* h = nullptr;
+    int rc = lane_state_for(b, l, b->n[c], &h);
+    if (rc) return rc;
+  }
+  return MQ_OK;
+}
+
+// Groups of the large circuits, their lanes (longest processing time first)
+// and device memory.
+static cudaError_t plan_groups(mq_batch* b) {
+  std::map<std::pair<int, int>, std::vector<int>> by;  // (n, ladder)
+  for (int c : b->large)
+    if (b->n[c] <= kGroupMaxQubits) by[{b->n[c], b->ladder[c]}].push_back(c);
+  std::vector<GroupCirc> table;
+  for (auto& [key, list] : by) {
+    std::stable_sort(list.begin(), list.end(), [&](int x, int y) { return b->depth[x] > b->depth[y]; });
+    const size_t most = std::max<size_t>(1, kGroupAmps >> key.first);
+    // groups of equal size, each with the whole range of depths
+    const size_t ng = (list.size() + most - 1) / most;
+    for (size_t g = 0; g < ng; ++g) {
+      mq_batch::Group G;
+      G.n = key.first;
+      G.ladder = key.second != 0;
+      G.first = (uint32_t)table.size();
+      for (size_t i = g; i < list.size(); i += ng) {
+        const int c = list[i];
+        G.circ.push_back(c);
+        table.push_back({b->mats_off[c], b->probs_off[c], (uint32_t)c, (uint32_t)b->depth[c]});
+      }
+      b->groups.push_back(std::move(G));
+    }
+  }
+  auto load = [&](const mq_batch::Group& G) {
+    uint64_t v = 0;
+    for (int c : G.circ) v += (uint64_t)std::max(1, b->depth[c]) << G.n;
+    return v;
+  };
+  b->lane_groups.resize(b->lanes);
+  std::vector<int> order(b->groups.size());
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return load(b->groups[x]) > load(b->groups[y]); });
+  std::vector<uint64_t> sum(b->lanes, 0);
+  std::vector<size_t> amps(b->lanes, 0);
+  for (int g : order) {
+    const int l = (int)(std::min_element(sum.begin(), sum.end()) - sum.begin());
+    b->lane_groups[l].push_back(g);
+    sum[l] += load(b->groups[g]);
+    amps[l] = std::max(amps[l], b->groups[g].circ.size() << b->groups[g].n);
+    b->zslots = std::max<size_t>(b->zslots, b->groups[g].circ.size() * group_blocks(b, b->groups[g].n));
+  }
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < 2; ++i) {
+    b->lane_buf[i].assign(b->lanes, nullptr);
+    for (int l = 0; l < b->lanes && e == cudaSuccess; ++l)
+      if (amps[l]) e = cudaMalloc(&b->lane_buf[i][l], amps[l] * sizeof(float2));
+  }
+  if (e == cudaSuccess && !table.empty()) e = cudaMalloc(&b->d_group, table.size() * sizeof(GroupCirc));
+  if (e == cudaSuccess && !table.empty())
+    e = cudaMemcpy(b->d_group, table.data(), table.size() * sizeof(GroupCirc), cudaMemcpyHostToDevice);
+  return e;
 }
 
 }  // namespace mq
@@ -406,20 +950,10 @@ int mq_batch_create(int device, void* stream, int n_circuits, const int32_t* n_q
     if (rc) { batch_free(b); return rc; }
   }
   if (!b->large.empty()) {
+    b->zblocks = (uint32_t)b->num_sms * 4;
     b->lanes = std::min<int>(lanes, (int)b->large.size());
-    b->lane_work.resize(b->lanes);
-    b->lane_state.resize(b->lanes);
-    // longest-processing-time assignment of circuits to lanes
-    std::vector<int> order = b->large;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-      return ((uint64_t)std::max(1, b->depth[x]) << b->n[x]) > ((uint64_t)std::max(1, b->depth[y]) << b->n[y]);
-    });
-    std::vector<uint64_t> load(b->lanes, 0);
-    for (int c : order) {
-      const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-      b->lane_work[l].push_back(c);
-      load[l] += (uint64_t)std::max(1, b->depth[c]) << b->n[c];
-    }
+    e = plan_groups(b);
+    if (e != cudaSuccess) return bail(e, "batch group setup");
     for (int l = 0; l < b->lanes; ++l) {
       cudaStream_t s;
       cudaEvent_t ev;
@@ -429,16 +963,15 @@ int mq_batch_create(int device, void* stream, int n_circuits, const int32_t* n_q
       e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
       if (e != cudaSuccess) return bail(e, "cudaEventCreate(lane)");
       b->lane_event.push_back(ev);
-      for (int c : b->lane_work[l]) {
-        mq_state* h = nullptr;
-        int rc = lane_state_for(b, l, b->n[c], &h);
-        if (rc) { batch_free(b); return rc; }
-      }
     }
     e = cudaEventCreateWithFlags(&b->fork_event, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(e, "cudaEventCreate(fork)");
-    b->zblocks = (uint32_t)b->num_sms * 4;
-    e = cudaMalloc(&b->d_zpart, (size_t)b->lanes * b->zblocks * sizeof(double));
+    {
+      int rc = plan_singles(b);
+      if (rc) { batch_free(b); return rc; }
+    }
+    b->zslots = std::max<size_t>(b->zslots, b->zblocks);
+    e = cudaMalloc(&b->d_zpart, (size_t)b->lanes * b->zslots * sizeof(double));
     if (e != cudaSuccess) return bail(e, "cudaMalloc(batch partials)");
   }
   *out = b;
@@ -465,7 +998,16 @@ int mq_batch_set_tiles(mq_batch* b, int tile_max, int passengers, int tile_min) 
   b->tile_max = tile_max;
   b->tile_pas = passengers;
   b->tile_min = tile_min;
-  return MQ_OK;
+  if (b->large.empty()) return MQ_OK;
+  MQ_TRY_BEGIN
+  DeviceGuard g(b->device);
+  int rc = plan_singles(b);
+  if (rc) {
+    b->tile_max = b->tile_min = 0;
+    b->tile_pas = -1;
+  }
+  return rc;
+  MQ_TRY_END
 }
 
 int mq_batch_run(mq_batch* b, const double* mats, float* probs_dev, double* z0_dev) {
