@@ -194,6 +194,23 @@ int mq_adjoint_layer_xor_async(mq_state* psi, mq_state* lam, const uint64_t* row
                                const int32_t* qubits, const double* mats, double* out_dev);
 
 /* ---- batched circuits (integrations/qiskit.py:505-514 runs them one by one) */
+/* Gate-stream fusion on the host (no device, no state): n_ops gates in order,
+ * gate i with code codes[i] (0..29: H I X Y Z S SDG T TDG SX RX RY RZ U1 U2 U3
+ * CNOT CH CZ CPHASE CRX CRY CRZ SWAP ISWAP XXPHASE YYPHASE ZZPHASE TOFFOLI
+ * FREDKIN), n_wires[i] entries of wires and n_params[i] of params (each list
+ * flat, in order).  Writes the fused segments to ints / doubles; used[0] and
+ * used[1] are the entries written (MQ_EUNSUPPORTED when a capacity is less).
+ * A segment of ints is one of
+ *   0 j m inverse                       QFT stage j of the wires [j, m)
+ *   1 k q[k]                            2x2 matrices (8 doubles each)
+ *   2 k (kind a b)[k]                   diagonal terms (8 doubles each)
+ *   3 c rows[n]                         GF(2) permutation
+ *   4 yy k (a b)[k]                     XX (yy = 0) or YY terms (1 double each)
+ *   5 k (n_controls controls target)[k] controlled 2x2 (8 doubles each). */
+int mq_fuse_stream(int n, int n_ops, const int32_t* codes, const int32_t* n_wires, const int32_t* wires,
+                   const int32_t* n_params, const double* params, int32_t* ints, int64_t ints_cap,
+                   double* doubles, int64_t doubles_cap, int64_t* used);
+
 /* A batch of layered circuits: circuit c has n_qubits[c] qubits (1..30) and
  * depth[c] layers, each a 2x2 on every qubit followed (ladder[c] != 0, or
  * ladder == NULL) by CNOT(0,1), ..., CNOT(n-2,n-1).  Circuits of <= 13 qubits

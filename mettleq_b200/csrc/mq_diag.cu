@@ -16,6 +16,7 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "mq_internal.cuh"
@@ -117,9 +118,27 @@ __global__ void __launch_bounds__(256) k_diag(V2<R>* __restrict__ st, const __gr
 }
 
 // ---------------------------------------------------------------- planner
+// at most N values in place (terms are copied while a plan is sought)
+template <typename T, int N>
+struct Few {
+  int n = 0;
+  T v[N];
+  void push_back(T x) { v[n++] = x; }
+  Few& operator=(std::initializer_list<T> l) {
+    n = 0;
+    for (const T& x : l) push_back(x);
+    return *this;
+  }
+  const T* begin() const { return v; }
+  const T* end() const { return v + n; }
+  size_t size() const { return (size_t)n; }
+  T& operator[](size_t i) { return v[i]; }
+  const T& operator[](size_t i) const { return v[i]; }
+};
 struct Term {
-  std::vector<int> bits;                   // global index bits, first = MSB of table index
-  std::vector<std::complex<double>> tab;   // 2^|bits| values
+  Few<int, 2> bits;                    // global index bits, first = MSB of table index
+  Few<std::complex<double>, 4> tab;    // 2^|bits| values
+  int lo = 0, hi = 0;                  // lowest and highest bit
 };
 
 struct PlannedLut {
@@ -163,44 +182,34 @@ static int build_terms(int n, int n_terms, const int32_t* kinds, const int32_t* 
     if (kind == MQ_DIAG_PHASE && std::fabs(th - M_PI) < 1e-15) tm.tab[1] = -1.0;
     tm.bits.push_back(n - 1 - a);
     if (two) tm.bits.push_back(n - 1 - b);
+    tm.lo = *std::min_element(tm.bits.begin(), tm.bits.end());
+    tm.hi = *std::max_element(tm.bits.begin(), tm.bits.end());
     terms.push_back(std::move(tm));
   }
   return MQ_OK;
 }
 
-static std::complex<double> term_value(const Term& tm, const std::vector<int>& pos, uint32_t x) {
-  uint32_t idx = 0;
-  const int k = (int)tm.bits.size();
-  for (int j = 0; j < k; ++j) {
-    const int gb = tm.bits[j];
-    int lp = (int)(std::find(pos.begin(), pos.end(), gb) - pos.begin());
-    const uint32_t bit = (x >> lp) & 1u;
-    idx |= bit << (k - 1 - j);
+// v[x] *= the term's value at x, where bit p of x is the global bit pos[p], for
+// every x.  Term by term over the whole table: an entry's factors multiply up
+// in the order of the terms, and a run of entries takes one factor.  (The
+// products are written out: std::complex checks each for infinities.)
+static void multiply_term(std::vector<std::complex<double>>& v, const Term& tm, const std::vector<int>& pos) {
+  auto at = [&](int bit) { return (int)(std::find(pos.begin(), pos.end(), bit) - pos.begin()); };
+  const int hi = at(tm.bits[0]), lo = tm.bits.size() == 2 ? at(tm.bits[1]) : -1;  // table index: bits[0] first
+  const size_t run = size_t(1) << (lo < 0 ? hi : std::min(hi, lo));
+  for (size_t x = 0; x < v.size(); x += run) {
+    const size_t i = lo < 0 ? (x >> hi) & 1u : (((x >> hi) & 1u) << 1) | ((x >> lo) & 1u);
+    const double fr = tm.tab[i].real(), fi = tm.tab[i].imag();
+    for (size_t k = x; k < x + run; ++k) {
+      const double re = v[k].real(), im = v[k].imag();
+      v[k] = {re * fr - im * fi, re * fi + im * fr};
+    }
   }
-  return tm.tab[idx];
 }
 
 static void finalize_lut(PlannedLut& L) {
-  const uint32_t sz = 1u << L.pos.size();
-  // table-local position of every member bit, found once
-  struct Local { int k, lp[2]; const std::complex<double>* tab; };
-  std::vector<Local> ms;
-  for (const Term* tm : L.members) {
-    Local m{(int)tm->bits.size(), {0, 0}, tm->tab.data()};
-    for (int j = 0; j < m.k; ++j)
-      m.lp[j] = (int)(std::find(L.pos.begin(), L.pos.end(), tm->bits[j]) - L.pos.begin());
-    ms.push_back(m);
-  }
-  L.vals.assign(sz, 1.0);
-  for (uint32_t x = 0; x < sz; ++x) {
-    std::complex<double> v = 1.0;
-    for (const Local& m : ms) {
-      uint32_t idx = 0;
-      for (int j = 0; j < m.k; ++j) idx |= ((x >> m.lp[j]) & 1u) << (m.k - 1 - j);
-      v *= m.tab[idx];
-    }
-    L.vals[x] = v;
-  }
+  L.vals.assign(size_t(1) << L.pos.size(), 1.0);
+  for (const Term* tm : L.members) multiply_term(L.vals, *tm, L.pos);
 }
 // Table values of a chosen plan (planning itself only sizes the tables).
 static void realize(std::vector<PlannedLut>& luts) {
@@ -213,21 +222,19 @@ static std::vector<PlannedLut> plan_luts(const std::vector<Term>& terms, int W) 
   std::vector<PlannedLut> luts;
   std::vector<int> local, far;
   for (size_t t = 0; t < terms.size(); ++t) {
-    auto [mn, mx] = std::minmax_element(terms[t].bits.begin(), terms[t].bits.end());
-    ((*mx - *mn) < W ? local : far).push_back((int)t);
+    (terms[t].hi - terms[t].lo < W ? local : far).push_back((int)t);
   }
   std::vector<bool> done(terms.size(), false);
   while (true) {
     int s = 1 << 30;
     for (int t : local)
-      if (!done[t]) s = std::min(s, *std::min_element(terms[t].bits.begin(), terms[t].bits.end()));
+      if (!done[t]) s = std::min(s, terms[t].lo);
     if (s == (1 << 30)) break;
     std::vector<const Term*> members;
     int hi = s;
     for (int t : local) {
       if (done[t]) continue;
-      auto [mn, mx] = std::minmax_element(terms[t].bits.begin(), terms[t].bits.end());
-      if (*mn >= s && *mx < s + W) { done[t] = true; members.push_back(&terms[t]); hi = std::max(hi, *mx); }
+      if (terms[t].lo >= s && terms[t].hi < s + W) { done[t] = true; members.push_back(&terms[t]); hi = std::max(hi, terms[t].hi); }
     }
     PlannedLut L;
     for (int b = s; b <= hi; ++b) L.pos.push_back(b);
@@ -257,6 +264,29 @@ static std::vector<PlannedLut> plan_luts(const std::vector<Term>& terms, int W) 
     luts.push_back(std::move(L));
   }
   return luts;
+}
+
+// Whether plan_luts(terms, W) would exceed `most` table entries or kMaxLuts
+// tables, where that shows without building it (no term wider than a window).
+static bool too_large(const std::vector<Term>& terms, int W, size_t most) {
+  std::vector<bool> done(terms.size(), false);
+  size_t entries = 0;
+  for (const Term& t : terms)
+    if (t.hi - t.lo >= W) return false;
+  for (int tables = 0;; ++tables) {
+    int s = 1 << 30;
+    for (size_t t = 0; t < terms.size(); ++t)
+      if (!done[t]) s = std::min(s, terms[t].lo);
+    if (s == (1 << 30)) return entries > most;
+    if (tables == kMaxLuts) return true;
+    int hi = s;
+    for (size_t t = 0; t < terms.size(); ++t)
+      if (!done[t] && terms[t].hi < s + W) {
+        done[t] = true;
+        hi = std::max(hi, terms[t].hi);
+      }
+    entries += size_t(1) << (hi - s + 1);
+  }
 }
 
 template <typename R>
@@ -301,6 +331,12 @@ static int launch_diag_pass(mq_state* h, const std::vector<PlannedLut>& in_luts)
   return MQ_OK;
 }
 
+int check_diag_terms(const mq_state* h, int n_terms, const int32_t* kinds, const int32_t* wires, const double* params) {
+  std::vector<Term> terms;
+  std::complex<double> scalar;
+  return build_terms(h->n, n_terms, kinds, wires, params, terms, scalar);
+}
+
 // The diagonal as contiguous-window tables for a tile-sweep epilogue (the
 // fused layer of mq_tile.cu): same factorisation as launch_diag_terms, with
 // the global phase folded into the first table.  out.n = -1 when no plan with
@@ -314,6 +350,7 @@ int plan_diag_windows(mq_state* h, int n_terms, const int32_t* kinds, const int3
   out = DiagWindows();
   out.n = -1;
   for (int W = 10; W >= 1; --W) {
+    if (too_large(terms, W, (size_t)std::max(max_entries, 0))) continue;
     std::vector<PlannedLut> luts = plan_luts(terms, W);
     size_t entries = 0;
     bool contig = true;
@@ -382,14 +419,14 @@ int plan_diag_register(mq_state* h, int n_terms, const int32_t* kinds, const int
   for (int b : cross) pos.push_back(b);
   const uint32_t nt = 1u << pos.size();
   std::vector<std::complex<double>> T(nt, scalar);
-  for (uint32_t x = 0; x < nt; ++x)
-    for (const Term& t : reg) T[x] *= term_value(t, pos, x);
+  for (const Term& t : reg) multiply_term(T, t, pos);
   // W: contiguous windows over the group terms
   std::vector<PlannedLut> luts;
   bool ok = false;
   for (int W = 10; W >= 1 && !ok; --W) {
-    luts = plan_luts(group, W);
     size_t entries = (nt / 16) * 17;
+    if ((int)entries > max_entries || too_large(group, W, (size_t)max_entries - entries)) continue;
+    luts = plan_luts(group, W);
     bool contig = true;
     for (auto& L : luts) {
       entries += lut_size(L);

@@ -294,6 +294,8 @@ int launch_cu2_list(mq_state* h, int n_gates, const int32_t* targets, const uint
 // Diagonal layers (mq_diag.cu)
 int launch_diag_terms(mq_state* h, int n_terms, const int32_t* kinds, const int32_t* wires,
                       const double* params);
+// MQ_EINVAL when a term is malformed.
+int check_diag_terms(const mq_state* h, int n_terms, const int32_t* kinds, const int32_t* wires, const double* params);
 // A diagonal factored into <= 8 tables indexed by contiguous index windows:
 // phase(x) = prod_w vals[off[w] + ((x >> shift[w]) & (2^nbits[w] - 1))]
 // (vals: re, im interleaved).  Planned by mq_diag.cu for tile epilogues.

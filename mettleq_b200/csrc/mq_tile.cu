@@ -2016,8 +2016,7 @@ int launch_layer(mq_state* h, const double* mats, const uint8_t* active, int n_t
   if (mats && !mats_dev && !active && (n_terms > 0 || euler_plain()) && euler_enabled(h)) {
     // validate the layer's own terms before anything is launched
     if (n_terms > 0) {
-      DiagWindows probe;
-      int rc = plan_diag_windows(h, n_terms, kinds, wires, params, 1, probe);
+      int rc = check_diag_terms(h, n_terms, kinds, wires, params);
       if (rc) return rc;
     }
     bool done = false;

@@ -28,11 +28,7 @@ def _ptr(a: np.ndarray):
 
 
 def _mats_array(n: int, mats) -> np.ndarray:
-    m = np.asarray(mats, dtype=np.complex128).reshape(n, 4)
-    out = np.empty((n, 8), dtype=np.float64)
-    out[:, 0::2] = m.real
-    out[:, 1::2] = m.imag
-    return np.ascontiguousarray(out)
+    return np.array(mats, dtype=np.complex128, order="C").reshape(n, 4).view(np.float64)
 
 
 def _pack_terms(terms):
@@ -41,15 +37,17 @@ def _pack_terms(terms):
     k = len(terms)
     if k == 0:
         return None, None, None
-    kinds = np.empty(k, dtype=np.int32)
+    kind, a, b, p = zip(*terms)
+    kinds = np.array(kind, dtype=np.int32)
     wires = np.empty(2 * k, dtype=np.int32)
+    wires[0::2] = a
+    wires[1::2] = b
     params = np.zeros((k, 8), dtype=np.float64)
-    for i, (kind, a, b, p) in enumerate(terms):
-        kinds[i] = int(kind)
-        wires[2 * i] = int(a)
-        wires[2 * i + 1] = int(b)
-        pp = list(p)
-        params[i, :len(pp)] = pp
+    if all(len(x) == 1 for x in p):
+        params[:, 0] = [x[0] for x in p]
+    else:
+        for i, x in enumerate(p):
+            params[i, :len(x)] = x
     return kinds, wires, params
 
 

@@ -28,11 +28,14 @@ basis change's sweeps carrying the ZZ terms) and one U(2) layer.
 """
 from __future__ import annotations
 
+import ctypes
 import math
+from itertools import chain
 from typing import Any, Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
 
+from . import _native as N
 from . import gates as G
 
 # kinds shared with the C ABI (include/mq.h)
@@ -330,14 +333,119 @@ def _mark_qft_stages(ops: List[dict]) -> List[dict]:
     return out
 
 
+# the gate codes of mq_fuse_stream
+GATE_NAMES = ("H", "I", "X", "Y", "Z", "S", "SDG", "T", "TDG", "SX", "RX", "RY", "RZ", "U1", "U2", "U3",
+              "CNOT", "CH", "CZ", "CPHASE", "CRX", "CRY", "CRZ", "SWAP", "ISWAP", "XXPHASE", "YYPHASE", "ZZPHASE",
+              "TOFFOLI", "FREDKIN")
+_CODES = {name: i for i, name in enumerate(GATE_NAMES)}
+_CODES.update({alias: _CODES[name] for alias, name in G.ALIASES.items()})
+# parameters of a diagonal term, by kind
+_TERM_PARAMS = (1, 1, 1, 1, 1, 1, 4, 8)
+
+
+def _native_segments(operations: Sequence[dict], n: int) -> Optional[List[Dict[str, Any]]]:
+    """The fused segments of ``fuse`` (before merging) from mq_fuse_stream, for
+    streams of ordinary gates; None for any other stream (pseudo-ops, other
+    spellings of names, values that are not plain numbers, malformed gates),
+    which the Python rules below handle or refuse.  One pass over the op
+    dicts builds the arrays; the per-gate work is native."""
+    if not (1 <= n <= 31):
+        return None
+    try:
+        codes = [_CODES[op["name"]] for op in operations]
+        wires = [op["wires"] for op in operations]
+        params = [op.get("parameters") or () for op in operations]
+        count = len(codes)
+        n_wires = np.fromiter(map(len, wires), np.int32, count)
+        n_params = np.fromiter(map(len, params), np.int32, count)
+        flat_w = np.fromiter(chain.from_iterable(wires), np.int32, int(n_wires.sum()))
+        flat_p = np.fromiter(chain.from_iterable(params), np.float64, int(n_params.sum()))
+        lib = N.lib()
+    except (KeyError, TypeError, ValueError, OverflowError, AttributeError, RuntimeError):
+        return None
+    code = np.array(codes, dtype=np.int32)
+    ints = np.empty(3 * count * (n + 8) + 16, dtype=np.int32)
+    doubles = np.empty(24 * count + 16, dtype=np.float64)
+    used = np.zeros(2, dtype=np.int64)
+
+    def ptr(a):
+        return a.ctypes.data_as(ctypes.c_void_p)
+
+    rc = lib.mq_fuse_stream(n, count, ptr(code), ptr(n_wires), ptr(flat_w), ptr(n_params), ptr(flat_p), ptr(ints),
+                            ints.size, ptr(doubles), doubles.size, ptr(used))
+    if rc != N.MQ_OK:
+        return None
+    return _decode(ints[:used[0]].tolist(), doubles[:used[1]].copy(), n)
+
+
+def _decode(v: List[int], d: np.ndarray, n: int) -> List[Dict[str, Any]]:
+    """The segments of mq_fuse_stream (include/mq.h) as layer dicts."""
+    out: List[Dict[str, Any]] = []
+    i = at = 0
+    mask = (1 << 32) - 1
+    while i < len(v):
+        kind = v[i]
+        if kind == 0:
+            out.append({"name": "_QFTSTAGE", "j": v[i + 1], "m": v[i + 2], "inverse": bool(v[i + 3])})
+            i += 4
+            continue
+        k = v[i + 1]
+        if kind == 1:
+            active = v[i + 2:i + 2 + k]
+            mats = np.tile(_EYE.reshape(1, 4), (n, 1))
+            mats[active] = d[at:at + 8 * k].view(np.complex128).reshape(k, 4)
+            out.append({"name": "_U2LISTLAYER", "mats": mats, "active": active})
+            i += 2 + k
+            at += 8 * k
+        elif kind == 2:
+            f = v[i + 2:i + 2 + 3 * k]
+            p = d[at:at + 8 * k].reshape(k, 8).tolist()
+            out.append({"name": "_DIAG", "terms": [(t, a, b, x[:_TERM_PARAMS[t]])
+                                                   for t, a, b, x in zip(f[0::3], f[1::3], f[2::3], p)]})
+            i += 2 + 3 * k
+            at += 8 * k
+        elif kind == 3:
+            out.append({"name": "_XORLAYER", "rows": [r & mask for r in v[i + 2:i + 2 + n]], "c": k & mask})
+            i += 2 + n
+        elif kind == 4:
+            k = v[i + 2]
+            f = v[i + 3:i + 3 + 2 * k]
+            out.append({"name": "_PAIRLAYER", "kind": "YY" if v[i + 1] else "XX", "bonds": list(zip(f[0::2], f[1::2])),
+                        "thetas": d[at:at + k].tolist()})
+            i += 3 + 2 * k
+            at += k
+        else:
+            gates = []
+            i += 2
+            for _ in range(k):
+                c = v[i]
+                gates.append((v[i + 1:i + 1 + c], v[i + 1 + c],
+                              d[at:at + 8].view(np.complex128).reshape(2, 2)))
+                i += 2 + c
+                at += 8
+            out.append({"name": "_CULIST", "gates": gates})
+    return out
+
+
 def fuse(operations: Sequence[dict], n: int, *, schedule: bool = True) -> List[Dict[str, Any]]:
+    if schedule:
+        fused = _native_segments(operations, n)
+        if fused is not None:
+            return fuse_layers(_merge(fused, n))
+    return _fuse_python(operations, n, schedule)
+
+
+def _fuse_python(operations: Sequence[dict], n: int, schedule: bool) -> List[Dict[str, Any]]:
+    """``fuse`` for every stream, and with the checks that name what is wrong
+    with a malformed one (6.0 ms for 1160 gates on 20 qubits, 0.96 ms by
+    mq_fuse_stream)."""
     ops = _mark_qft_stages(decompose(normalize(operations, n)))
     if schedule:
         ops = dependency_schedule(ops)
     fused: List[Dict[str, Any]] = []
     i = 0
-    N = len(ops)
-    while i < N:
+    count = len(ops)
+    while i < count:
         op = ops[i]
         name = op["name"]
         if name == "_QFTSTAGE":
@@ -347,7 +455,7 @@ def fuse(operations: Sequence[dict], n: int, *, schedule: bool = True) -> List[D
         if len(op.get("wires", [])) == 1:
             j = i
             per_wire: Dict[int, np.ndarray] = {}
-            while j < N and len(ops[j].get("wires", [])) == 1 and ops[j]["name"] != "_QFTSTAGE":
+            while j < count and len(ops[j].get("wires", [])) == 1 and ops[j]["name"] != "_QFTSTAGE":
                 q = ops[j]["wires"][0]
                 per_wire[q] = _single_matrix(ops[j]) @ per_wire.get(q, _EYE)
                 j += 1
@@ -357,7 +465,7 @@ def fuse(operations: Sequence[dict], n: int, *, schedule: bool = True) -> List[D
         if name in DIAG_TWO:
             terms = []
             j = i
-            while j < N and (ops[j]["name"] in DIAG_TWO):
+            while j < count and (ops[j]["name"] in DIAG_TWO):
                 terms.extend(diag_terms_of(ops[j], n))
                 j += 1
             fused.append({"name": "_DIAG", "terms": terms})
@@ -365,7 +473,7 @@ def fuse(operations: Sequence[dict], n: int, *, schedule: bool = True) -> List[D
             continue
         if name in AFFINE:
             j = i
-            while j < N and ops[j]["name"] in AFFINE:
+            while j < count and ops[j]["name"] in AFFINE:
                 j += 1
             rows, c = affine_of(ops[i:j], n)
             fused.append({"name": "_XORLAYER", "rows": rows, "c": c})
@@ -377,7 +485,7 @@ def fuse(operations: Sequence[dict], n: int, *, schedule: bool = True) -> List[D
             # (shaders/pauli_pair.py:32-64)
             bonds, thetas = [], []
             j = i
-            while j < N and ops[j]["name"] == name:
+            while j < count and ops[j]["name"] == name:
                 bonds.append(tuple(ops[j]["wires"]))
                 thetas.append(float(ops[j]["parameters"][0]))
                 j += 1
@@ -388,7 +496,7 @@ def fuse(operations: Sequence[dict], n: int, *, schedule: bool = True) -> List[D
         if name in CONTROLLED:
             gates = []
             j = i
-            while j < N and ops[j]["name"] in CONTROLLED:
+            while j < count and ops[j]["name"] in CONTROLLED:
                 w = ops[j]["wires"]
                 gates.append((list(w[:-1]), w[-1], G.controlled_target_matrix(ops[j]["name"], ops[j]["parameters"])))
                 j += 1
