@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(kZThreads) k_pauli_z(const V2<R>* __restrict__
 // every word there (two products per pair).  Sums per word and thread stay in
 // shared memory.  Bound by the float64 work (16 products per 16 amplitudes
 // and word) and the float32 -> float64 conversions of every window; 25
-// qubits, 25 X words: 25 passes of 135 us before, three of 117 us on average now.
+// qubits, 25 X words: 25 passes of 135 us before, three of 79 us on average now (117 with every word through the switch).
 constexpr int kTileWords = 24;
 constexpr int kTileWins = 6;
 constexpr int kPauliLT = 7;
@@ -566,6 +566,7 @@ struct PauliWin {
   uint32_t s_reg[4], s_grp[8], g_grp[8];
   uint16_t w0, w1;  // words [w0, w1) of the window
   uint32_t zs;      // Z letters of its words outside it (0: signs need no index)
+  uint8_t one[4];   // word X on the window's bit k alone, no Z letters; 0xff: none
 };
 struct PauliTileWord {
   uint32_t z;         // Z mask outside the window (index bits)
@@ -689,6 +690,25 @@ __global__ void __launch_bounds__(1 << kPauliLT, 4) k_pauli_tile(const V2<R>* __
         // converted once here, not again for every word
 #pragma unroll
         for (int r = 0; r < 16; ++r) asm volatile("" : "+d"(ar[r]), "+d"(ai[r]));
+        // single X letters (a transverse field) without the switch below
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t w = W.one[k];
+          if (w == 0xffu) continue;
+          double s[4];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int r = ((j >> k) << (k + 1)) | (j & ((1 << k) - 1)), r1 = r | (1 << k);
+            if (j < 2) {
+              s[j] = ar[r] * ar[r1];
+              s[2 + j] = ai[r] * ai[r1];
+            } else {
+              s[j & 1] = fma(ar[r], ar[r1], s[j & 1]);
+              s[2 + (j & 1)] = fma(ai[r], ai[r1], s[2 + (j & 1)]);
+            }
+          }
+          acc[w * NT + tid] += (s[0] + s[1]) + (s[2] + s[3]);
+        }
         for (int w = W.w0; w < W.w1; ++w) {
           const PauliTileWord& D = P.word[w];
           double s;
@@ -1082,8 +1102,11 @@ static int pauli_launch(mq_state* h, int n_words, const uint64_t* xmask, const u
   for (size_t sw = 0; sw < sweeps.size(); ++sw) {
     std::vector<std::pair<int, int>> todo;  // (window, word)
     for (size_t k = 0; k < wins.size(); ++k)
-      if (wins[k].sweep == (int)sw)
+      if (wins[k].sweep == (int)sw) {
+        auto single = [&](int w) { return zmask[w] == 0 && (xmask[w] & (xmask[w] - 1)) == 0; };
+        std::stable_partition(in_win[k].begin(), in_win[k].end(), single);
         for (int w : in_win[k]) todo.push_back({(int)k, w});
+      }
     const uint32_t n_tiles = (uint32_t)(h->dim() >> M);
     const uint32_t grid = std::min<uint32_t>(n_tiles, (uint32_t)h->num_sms * 4);
     const size_t most = std::min<size_t>(kTileWords, part_cap / grid);
@@ -1101,6 +1124,7 @@ static int pauli_launch(mq_state* h, int n_words, const uint64_t* xmask, const u
           if (P.n_win == kTileWins) break;
           open = todo[i].first;
           PauliWin& D = P.win[P.n_win++];
+          std::memset(D.one, 0xff, sizeof(D.one));
           D.w0 = (uint16_t)idx.size();
           auto phys = [c64](uint32_t v) -> uint32_t { return c64 ? (v ^ ((v >> 3) & 0xEu)) : (v ^ ((v >> 3) & 7u)); };
           int j = 0, r = 0;
@@ -1125,9 +1149,15 @@ static int pauli_launch(mq_state* h, int n_words, const uint64_t* xmask, const u
           if (odd(r & zr)) T.sgn |= (uint16_t)(1u << r);
         T.z = (uint32_t)zmask[w] & ~W.mask;
         T.imag = odd(xmask[w] & zmask[w]) ? 1 : 0;
+        PauliWin& D = P.win[P.n_win - 1];
+        if (zmask[w] == 0 && (T.x & (T.x - 1)) == 0 && D.one[__builtin_ctz(T.x)] == 0xff && D.w0 == idx.size()) {
+          // single X letters come first in the window's list (a repeated one ends them)
+          D.one[__builtin_ctz(T.x)] = (uint8_t)idx.size();
+          D.w0 = (uint16_t)(idx.size() + 1);
+        }
         idx.push_back(w);
-        P.win[P.n_win - 1].w1 = (uint16_t)idx.size();
-        P.win[P.n_win - 1].zs |= T.z;
+        D.w1 = (uint16_t)idx.size();
+        D.zs |= T.z;
       }
       P.n_words = (uint8_t)idx.size();
       const size_t smem = (h->amp_bytes() << M) + sizeof(double) * idx.size() * (1u << kPauliLT);

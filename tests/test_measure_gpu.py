@@ -86,4 +86,6 @@ def test_pauli_words_over_every_kernel_of_the_split(n, dtype):
     assert np.array_equal(sv.expval_pauli(words), got)
     one = int(rng.integers(len(words)))
     assert sv.expval_pauli([words[one]])[0] == got[one]  # a word's bits do not depend on the others
+    twice = [w for w in words for _ in range(2)]
+    assert np.array_equal(sv.expval_pauli(twice), np.repeat(got, 2))
     sv.close()
