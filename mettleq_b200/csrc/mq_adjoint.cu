@@ -219,7 +219,13 @@ __device__ unsigned int g_adj_fault;
 // pair, and writes them back as two TMA stores; every wait is bounded
 // (kTmaWaitNs), and a CTA whose tile does not arrive sets g_adj_fault and
 // returns as a whole.
-template <typename R, int M, int LR, int LT, bool TMA>
+//
+// ROLL: one copy of the phase code for all phases, the phase's sums moved in and
+// out of the registers of its index.  With three phases their copies run out of
+// the instruction cache (a fifth of the stalls); 24 qubits: the 10-target sweep
+// 220 -> 184 us with ROLL, but the two-phase sweeps 133 -> 140 us, so these keep
+// the copies.
+template <typename R, int M, int LR, int LT, bool TMA, bool ROLL>
 __global__ void __launch_bounds__(1 << LT)
 k_adj(V2<R>* psi, V2<R>* lam, const __grid_constant__ AdjParams P, double* __restrict__ partials) {
   using T = V2<R>;
@@ -377,13 +383,14 @@ k_adj(V2<R>* psi, V2<R>* lam, const __grid_constant__ AdjParams P, double* __res
       cp_async_wait<1>();
       __syncthreads();
     }
-#pragma unroll
-    for (int ph = 0; ph < MAXPH; ++ph) {
-      if (ph >= P.n_phases) break;
-      const AdjPhase& D = P.ph[ph];
+    // one phase on the tile pair: its sums go to sum[slot]
+    auto phase = [&](const AdjPhase& D, R (&sum)[LR][3]) {
       uint32_t sreg[LR];
 #pragma unroll
       for (int k = 0; k < LR; ++k) sreg[k] = D.s_reg[k];
+      // ROLL (complex64): with tile bit 0 in register slot 0, amplitudes r, r+1
+      // are one 16-byte chunk
+      const bool pair = ROLL && sreg[0] == 1u;
 #pragma unroll
       for (int g = 0; g < GPT; ++g) {
         const uint32_t q = (uint32_t)tid + (uint32_t)g * NT;
@@ -391,21 +398,46 @@ k_adj(V2<R>* psi, V2<R>* lam, const __grid_constant__ AdjParams P, double* __res
 #pragma unroll
         for (int j = 0; j < M - LR; ++j)
           if ((q >> j) & 1) sq ^= D.s_grp[j];
+        if (pair) {
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          a[r] = cp[sq ^ xsel<LR>(r, sreg)];
-          b[r] = cl[sq ^ xsel<LR>(r, sreg)];
+          for (int r = 0; r < NR; r += 2) {
+            const float4 v = *reinterpret_cast<const float4*>(cp + (sq ^ xsel<LR>(r, sreg)));
+            const float4 w = *reinterpret_cast<const float4*>(cl + (sq ^ xsel<LR>(r, sreg)));
+            a[r] = mk<R>((R)v.x, (R)v.y);
+            a[r + 1] = mk<R>((R)v.z, (R)v.w);
+            b[r] = mk<R>((R)w.x, (R)w.y);
+            b[r + 1] = mk<R>((R)w.z, (R)w.w);
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            a[r] = cp[sq ^ xsel<LR>(r, sreg)];
+            b[r] = cl[sq ^ xsel<LR>(r, sreg)];
+          }
         }
-        adj_slot<R, LR, 0>(a, b, D.slot[0], acc[ph][0]);
-        if constexpr (LR > 1) adj_slot<R, LR, 1>(a, b, D.slot[1], acc[ph][1]);
-        if constexpr (LR > 2) adj_slot<R, LR, 2>(a, b, D.slot[2], acc[ph][2]);
-        if constexpr (LR > 3) adj_slot<R, LR, 3>(a, b, D.slot[3], acc[ph][3]);
+        adj_slot<R, LR, 0>(a, b, D.slot[0], sum[0]);
+        if constexpr (LR > 1) adj_slot<R, LR, 1>(a, b, D.slot[1], sum[1]);
+        if constexpr (LR > 2) adj_slot<R, LR, 2>(a, b, D.slot[2], sum[2]);
+        if constexpr (LR > 3) adj_slot<R, LR, 3>(a, b, D.slot[3], sum[3]);
+        if (pair) {
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          if (P.store_psi) cp[sq ^ xsel<LR>(r, sreg)] = a[r];
-          cl[sq ^ xsel<LR>(r, sreg)] = b[r];
+          for (int r = 0; r < NR; r += 2) {
+            if (P.store_psi)
+              *reinterpret_cast<float4*>(cp + (sq ^ xsel<LR>(r, sreg))) =
+                  make_float4((float)a[r].x, (float)a[r].y, (float)a[r + 1].x, (float)a[r + 1].y);
+            *reinterpret_cast<float4*>(cl + (sq ^ xsel<LR>(r, sreg))) =
+                make_float4((float)b[r].x, (float)b[r].y, (float)b[r + 1].x, (float)b[r + 1].y);
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            if (P.store_psi) cp[sq ^ xsel<LR>(r, sreg)] = a[r];
+            cl[sq ^ xsel<LR>(r, sreg)] = b[r];
+          }
         }
       }
+    };
+    auto phase_end = [&](int ph) {
       // TMA: the tile's last shared-memory writes become visible to the
       // async proxy (the stores that read them, the load that overwrites)
       if constexpr (TMA)
@@ -418,6 +450,37 @@ k_adj(V2<R>* psi, V2<R>* lam, const __grid_constant__ AdjParams P, double* __res
           bulk_wait_read();
           tma_issue(next, cb ^ 1);
         }
+      }
+    };
+    if constexpr (ROLL) {
+#pragma unroll 1
+      for (int ph = 0; ph < P.n_phases; ++ph) {
+        R sum[LR][3];
+#pragma unroll
+        for (int p = 0; p < MAXPH; ++p)
+          if (ph == p) {
+#pragma unroll
+            for (int k = 0; k < LR; ++k)
+#pragma unroll
+              for (int e = 0; e < 3; ++e) sum[k][e] = acc[p][k][e];
+          }
+        phase(P.ph[ph], sum);
+#pragma unroll
+        for (int p = 0; p < MAXPH; ++p)
+          if (ph == p) {
+#pragma unroll
+            for (int k = 0; k < LR; ++k)
+#pragma unroll
+              for (int e = 0; e < 3; ++e) acc[p][k][e] = sum[k][e];
+          }
+        phase_end(ph);
+      }
+    } else {
+#pragma unroll
+      for (int ph = 0; ph < MAXPH; ++ph) {
+        if (ph >= P.n_phases) break;
+        phase(P.ph[ph], acc[ph]);
+        phase_end(ph);
       }
     }
     if constexpr (TMA) {
@@ -583,9 +646,9 @@ int take_adj_fault(mq_state* h, bool* fault) {
   return MQ_OK;
 }
 
-template <typename R, int M, int LR, int LT, bool TMA>
+template <typename R, int M, int LR, int LT, bool TMA, bool ROLL = false>
 static int launch_adj_t(mq_state* psi, mq_state* lam, const AdjParams& P0, double* partials, uint32_t* grid_out) {
-  auto kern = k_adj<R, M, LR, LT, TMA>;
+  auto kern = k_adj<R, M, LR, LT, TMA, ROLL>;
   size_t smem = 4 * sizeof(V2<R>) * (size_t(1) << M);
   AdjParams P = P0;
   if constexpr (TMA) {
@@ -641,6 +704,10 @@ static int dispatch_adj_lr(mq_state* psi, mq_state* lam, const AdjParams& P, dou
       constexpr int L = (MM) < LRT ? (MM) : LRT;                                     \
       constexpr int LTMAX = LRT == 3 ? 8 : 7;                                        \
       constexpr int LT = ((MM) - L) < LTMAX ? ((MM) - L) : LTMAX;                    \
+      if constexpr ((MM) >= 10 && LRT == 4) {                                        \
+        if (P.tma.ndim && P.n_phases >= 3)                                           \
+          return launch_adj_t<R, MM, L, LT, true, true>(psi, lam, P, partials, grid); \
+      }                                                                              \
       if constexpr ((MM) >= 10) {                                                    \
         if (P.tma.ndim) return launch_adj_t<R, MM, L, LT, true>(psi, lam, P, partials, grid); \
       }                                                                              \
