@@ -977,16 +977,15 @@ k_tile(const V2<R>* src, V2<R>* dst, const __grid_constant__ PT P) {
         // to their output slots, and the tile leaves as one TMA store to
         // output tile `tile`.  complex128, 25 qubits: 314 us for the low
         // sweep against 364 us with per-thread stores
-        float4* c4w = reinterpret_cast<float4*>(cur);
         float4 v[CPT];
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
           const uint32_t l0 = cl_in ^ epi_at ^ chunk_cols<LT, LCH, CB>(k, ecols);
-          const uint32_t ch = l0 >> CB;
-          const float4 w = c4w[ch ^ ((ch >> 3) & 7u)];
+          const float4 w = *reinterpret_cast<const float4*>(cur + amp_slot<R>(CB == 1 ? l0 & ~1u : l0));
           v[k] = (CB == 1 && (l0 & 1u)) ? make_float4(w.z, w.w, w.x, w.y) : w;
         }
         __syncthreads();
+        float4* c4w = reinterpret_cast<float4*>(cur);
 #pragma unroll
         for (int k = 0; k < CPT; ++k) c4w[slot(k)] = v[k];
         fence_proxy_async_smem();
