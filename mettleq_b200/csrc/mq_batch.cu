@@ -41,19 +41,24 @@ struct SmallCircuit {
 
 __device__ __forceinline__ uint32_t bslot(uint32_t i) { return i ^ ((i >> 3) & 0xEu); }
 
-__device__ __forceinline__ float2 cmac2f(float2 u0, float2 x0, float2 u1, float2 x1) {
-  float2 r;
-  r.x = fmaf(u0.x, x0.x, fmaf(-u0.y, x0.y, fmaf(u1.x, x1.x, -u1.y * x1.y)));
-  r.y = fmaf(u0.x, x0.y, fmaf(u0.y, x0.x, fmaf(u1.x, x1.y, u1.y * x1.x)));
-  return r;
+// u0 x0 + u1 x1 on the paired FP32 instructions, the entries given as
+// (u.x, u.x, -u.y, u.y).  Both components take the rounding steps of
+//   fma(u0.x, x0.x, fma(-u0.y, x0.y, fma(u1.x, x1.x, -u1.y x1.y)))
+//   fma(u0.x, x0.y, fma(u0.y, x0.x, fma(u1.x, x1.y, u1.y x1.x))).
+__device__ __forceinline__ float2 cmac2p(float4 u0, float2 x0, float4 u1, float2 x1) {
+  const float2 s0 = make_float2(x0.y, x0.x), s1 = make_float2(x1.y, x1.x);
+  return __ffma2_rn(x0, make_float2(u0.x, u0.y),
+                    __ffma2_rn(s0, make_float2(u0.z, u0.w),
+                               __ffma2_rn(x1, make_float2(u1.x, u1.y), __fmul2_rn(s1, make_float2(u1.z, u1.w)))));
 }
 
 template <int NT>
 __global__ void __launch_bounds__(NT) k_batch_small(const SmallCircuit* __restrict__ circ, uint32_t n_circ,
                                                     const double* __restrict__ mats, float* __restrict__ probs,
-                                                    double* __restrict__ z0, uint32_t* __restrict__ next) {
+                                                    double* __restrict__ z0, uint32_t* __restrict__ next,
+                                                    uint32_t half) {
   extern __shared__ __align__(16) float2 sm[];
-  __shared__ float2 um[kSmallMax][4];
+  __shared__ float4 um[kSmallMax][4];  // an entry u as (u.x, u.x, -u.y, u.y)
   __shared__ uint32_t cid;
   __shared__ double zred[NT / 32];
   const int tid = threadIdx.x;
@@ -67,13 +72,14 @@ __global__ void __launch_bounds__(NT) k_batch_small(const SmallCircuit* __restri
     const int n = (int)C.n;
     const uint32_t E = 1u << n;
     float2* a = sm;
-    float2* b = sm + (1u << kSmallMax);
+    float2* b = sm + half;
     for (uint32_t i = tid; i < E; i += NT) a[bslot(i)] = make_float2(i == 0 ? 1.f : 0.f, 0.f);
     for (uint32_t l = 0; l < C.depth; ++l) {
       __syncthreads();
       for (int j = tid; j < n * 4; j += NT) {
         const double* m = mats + C.mats_off + ((size_t)l * n * 4 + j) * 2;
-        um[j >> 2][j & 3] = make_float2((float)m[0], (float)m[1]);
+        const float x = (float)m[0], y = (float)m[1];
+        um[j >> 2][j & 3] = make_float4(x, x, -y, y);
       }
       __syncthreads();
       // 2x2 on every qubit, four index bits per register pass; the last pass
@@ -93,13 +99,13 @@ __global__ void __launch_bounds__(NT) k_batch_small(const SmallCircuit* __restri
             const int bit = lo + k;
             if (k >= nb || bit < g0) continue;
             const int q = n - 1 - bit;
-            const float2 u00 = um[q][0], u01 = um[q][1], u10 = um[q][2], u11 = um[q][3];
+            const float4 u[4] = {um[q][0], um[q][1], um[q][2], um[q][3]};
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
               if ((r & (1 << k)) || r >= (1 << nb)) continue;
               const float2 x0 = v[r], x1 = v[r | (1 << k)];
-              v[r] = cmac2f(u00, x0, u01, x1);
-              v[r | (1 << k)] = cmac2f(u10, x0, u11, x1);
+              v[r] = cmac2p(u[0], x0, u[1], x1);
+              v[r | (1 << k)] = cmac2p(u[2], x0, u[3], x1);
             }
           }
 #pragma unroll
@@ -178,10 +184,8 @@ constexpr int kSweepThreads = 256;
 constexpr int kSweepCtas = 3;  // 80 registers a thread: 4.68 ms a batch run; 4.90 with 2 CTAs, 5.51 with 4
 
 // One phase: 16 amplitudes differing in tile bits [4P, 4P + 4), the gates of
-// the first `cnt` of these bits in ascending order.  um: every matrix entry u
-// as the pairs (u.x, u.x), (-u.y, u.y), so that a component pair of cmac2f is
-// four paired FP32 instructions in its order (the same roundings): 5.19 -> 4.98
-// ms a batch run.
+// the first `cnt` of these bits in ascending order.  (Scalar FP32 instructions
+// instead of cmac2p: 5.19 against 4.98 ms a batch run.)
 template <int P>
 __device__ __forceinline__ void group_phase(float2* tile, uint32_t tid, int cnt, const float4 (*um)[4]) {
   float2 a[16];
@@ -199,23 +203,13 @@ __device__ __forceinline__ void group_phase(float2* tile, uint32_t tid, int cnt,
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (k >= cnt) break;
-    float2 u[4][2];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 q = um[k][j];
-      u[j][0] = make_float2(q.x, q.y);
-      u[j][1] = make_float2(q.z, q.w);
-    }
+    const float4 u[4] = {um[k][0], um[k][1], um[k][2], um[k][3]};
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
       if (r & (1 << k)) continue;
       const float2 x0 = a[r], x1 = a[r | (1 << k)];
-      const float2 s0 = make_float2(x0.y, x0.x), s1 = make_float2(x1.y, x1.x);
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        a[j ? (r | (1 << k)) : r] =
-            __ffma2_rn(x0, u[2 * j][0],
-                       __ffma2_rn(s0, u[2 * j][1], __ffma2_rn(x1, u[2 * j + 1][0], __fmul2_rn(s1, u[2 * j + 1][1]))));
+      a[r] = cmac2p(u[0], x0, u[1], x1);
+      a[r | (1 << k)] = cmac2p(u[2], x0, u[3], x1);
     }
   }
   if constexpr (P == 0) {
@@ -337,7 +331,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_group_first(const __grid_cons
   __shared__ float2 col[32][2];  // by gate order
   const uint32_t tid = threadIdx.x;
   const int n = P.n;
-  // a gate on amplitudes (v, 0): the rounding of cmac2f with x1 = 0
+  // a gate on amplitudes (v, 0): the rounding of cmac2p with x1 = 0
   auto times = [](float2 u, float2 v) { return make_float2(fmaf(u.x, v.x, -u.y * v.y), fmaf(u.x, v.y, u.y * v.x)); };
   uint32_t have = 0xffffffffu;
   for (uint32_t t = blockIdx.x; t < P.n_tiles; t += gridDim.x) {
@@ -597,15 +591,22 @@ static int lane_state_for(mq_batch* b, int lane, int n, mq_state** out) {
 
 template <int NT>
 static int launch_small(mq_batch* b, float* probs, double* z0, bool configure) {
-  const size_t smem = 2 * sizeof(float2) * (size_t(1) << kSmallMax);
-  if (configure) {
-    MQ_CUDA(cudaFuncSetAttribute(k_batch_small<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (configure) {  // the limit is the kernel's, not the batch's: always the largest
+    MQ_CUDA(cudaFuncSetAttribute(k_batch_small<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(2 * sizeof(float2) << kSmallMax)));
     return MQ_OK;
   }
+  // two buffers of the widest circuit: a batch of up to 12 qubits has two and
+  // more CTAs on an SM (200 circuits of 6 to 12 qubits: 85 -> 78 us, with cmac2p)
+  int widest = 1;
+  for (int c : b->small) widest = std::max(widest, (int)b->n[c]);
+  const uint32_t half = 1u << widest;
+  const size_t smem = 2 * sizeof(float2) * (size_t)half;
   int bps = 0;
   MQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_batch_small<NT>, NT, smem));
   const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(b->small.size(), (uint64_t)b->num_sms * std::max(1, bps)));
-  k_batch_small<NT><<<grid, NT, smem, b->stream>>>(b->d_small, (uint32_t)b->small.size(), b->d_mats, probs, z0, b->d_next);
+  k_batch_small<NT><<<grid, NT, smem, b->stream>>>(b->d_small, (uint32_t)b->small.size(), b->d_mats, probs, z0, b->d_next,
+                                             half);
   MQ_LAUNCHED("k_batch_small");
   return MQ_OK;
 }
@@ -780,13 +781,11 @@ static int record_batch(mq_batch* b, float* probs, double* z0) {
 // 2^21, 4.68 with 2^22, 4.80 with 2^23.
 constexpr size_t kGroupAmps = size_t(1) << 22;
 
-
 // The large circuits that run one by one, all of them with a tile plan set by
 // mq_batch_set_tiles, else those of 24 qubits and more, where the general
-// sweeps with TMA tiles are as fast (24 qubits, 6
-// circuits: 12.5 ms both; 23 qubits, 8: 8.6 against 8.2 ms in groups): their
-// lanes (longest processing time
-// first) and the lanes' states, with the tile plan set so far.
+// sweeps with TMA tiles are as fast (24 qubits, 6 circuits: 12.5 ms both; 23
+// qubits, 8 circuits: 8.6 against 8.2 ms in groups): their lanes (longest
+// processing time first) and the lanes' states, with the tile plan set so far.
 constexpr int kGroupMaxQubits = 23;
 static int plan_singles(mq_batch* b) {
   for (auto& m : b->lane_state)
