@@ -675,5 +675,30 @@ def expected_sweeps(layer: dict, n: int, dtype: str = "complex64") -> int:
         cnt = layer["j_end"] - layer["j_begin"]
         return 1 if cnt + pas <= tmax else -(-cnt // (tmax - pas))
     if name == "_CULIST":
-        return max(1, len(layer["gates"]))
+        return _controlled_sweeps([n - 1 - t for _, t, _ in layer["gates"]], n, tmax, pas)
     return 1
+
+
+def _controlled_sweeps(bits: List[int], n: int, tmax: int, pas: int) -> int:
+    """Sweeps of a controlled-gate list with these target bits (mq_tile.cu
+    launch_cu2_list): gates in order while their targets fit a tile, four to a
+    phase, six phases and 16 gates to a sweep."""
+    sweeps, i = 0, 0
+    while i < len(bits):
+        sweeps += 1
+        tile: set = set()
+        phase: set = set()
+        phases = in_phase = gates = 0
+        while i < len(bits) and gates < 16:
+            b = bits[i]
+            more = tile | {b}
+            if tile and len(more | set(range(min(max(pas, 1), min(more))))) > tmax:
+                break
+            if not phases or in_phase == min(4, n) or b in phase:
+                if phases == 6:
+                    break
+                phases, in_phase, phase = phases + 1, 0, set()
+            in_phase += 1
+            phase.add(b)
+            tile, gates, i = more, gates + 1, i + 1
+    return max(1, sweeps)
