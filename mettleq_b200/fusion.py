@@ -428,6 +428,8 @@ def _decode(v: List[int], d: np.ndarray, n: int) -> List[Dict[str, Any]]:
 
 
 def fuse(operations: Sequence[dict], n: int, *, schedule: bool = True) -> List[Dict[str, Any]]:
+    if not isinstance(operations, (list, tuple)):
+        operations = list(operations)  # read more than once below
     if schedule:
         fused = _native_segments(operations, n)
         if fused is not None:

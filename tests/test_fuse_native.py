@@ -81,6 +81,12 @@ def test_other_spellings_and_values_are_accepted_as_before(ops):
         _same(a, b)
 
 
+@pytest.mark.parametrize("name", ["H", "h"])
+def test_an_iterator_of_gates_is_read_once(name):
+    ops = [{"name": name, "wires": [q], "parameters": []} for q in range(3)]
+    assert [L["active"] for L in F.fuse(iter(ops), 3)] == [[0, 1, 2]]
+
+
 @pytest.mark.parametrize("op", [
     {"name": "RX", "wires": [0], "parameters": []}, {"name": "H", "wires": [0, 1]}, {"name": "CNOT", "wires": [1, 1]},
     {"name": "H", "wires": [3]}, {"name": "H", "wires": [-1]}, {"name": "H", "wires": [1 << 40]}, {"name": "FOO", "wires": [0]}])
