@@ -183,6 +183,8 @@ __device__ __forceinline__ uint32_t nib_index(uint32_t tid, uint32_t r) {
 constexpr int kSweepThreads = 256;
 constexpr int kSweepCtas = 3;  // 80 registers a thread: 4.68 ms a batch run; 4.90 with 2 CTAs, 5.51 with 4
 
+constexpr size_t kSweepSmem = 2 * 4096 * sizeof(float2);
+
 // One phase: 16 amplitudes differing in tile bits [4P, 4P + 4), the gates of
 // the first `cnt` of these bits in ascending order.  (Scalar FP32 instructions
 // instead of cmac2p: 5.19 against 4.98 ms a batch run.)
@@ -229,76 +231,90 @@ __device__ __forceinline__ void group_phase(float2* tile, uint32_t tid, int cnt,
 // the write-back (an output tile reads one input tile).  Else cnt <= 8 high
 // targets in tile bits [4, 4 + cnt) over the passengers 0-3; the tile's
 // remaining bits are the index bits from 4 up, so a run is 2^(12 - cnt)
-// amplitudes.  In place unless the ladder permutes.
+// amplitudes.  In place unless the ladder permutes.  The next tile and its
+// matrices are loaded while this one is worked on: 24 warps an SM did not cover
+// the wait (4.69 -> 4.56 ms a batch run).
 template <bool LOW>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_group_sweep(const __grid_constant__ GroupSweep P) {
-  __shared__ __align__(16) float2 tile[4096];
-  __shared__ float4 um[12][4];  // by tile bit
+  extern __shared__ __align__(16) float2 tiles[];  // two buffers of 4096
+  __shared__ float4 um[2][12][4];                  // by buffer, tile bit
+  __shared__ double2 raw[48];                      // the next tile's matrices as they are in memory
   uint32_t tid = threadIdx.x;
   const int n = P.n, cnt = P.cnt, pas = 12 - cnt;
-  uint32_t have = 0xffffffffu;
-  for (uint32_t t = blockIdx.x; t < P.n_tiles; t += gridDim.x) {
-    // keeps the per-chunk addresses from being held (spilled) across tiles
-    asm volatile("" : "+r"(tid));
-    const uint32_t cid = t >> (n - 12);
-    const uint32_t h = t & ((1u << (n - 12)) - 1u);
-    const size_t state = (size_t)cid << n;
-    uint32_t base;  // of the input tile
+  // consecutive chunks of a tile are consecutive in memory: chunk order over
+  // (passengers, targets), tile-local order (passengers 0-3, targets, other
+  // passengers)
+  auto local_of = [&](uint32_t i) -> uint32_t {
+    if constexpr (LOW) return i;
+    const uint32_t low = i & 15u, mid = (i >> 4) & ((1u << (pas - 4)) - 1u), tg = i >> pas;
+    return low | (tg << 4) | (mid << (4 + cnt));
+  };
+  auto offset_of = [&](uint32_t i) -> uint32_t {
+    if constexpr (LOW) return i;
+    else return (i & ((1u << pas) - 1u)) | ((i >> pas) << P.start);
+  };
+  auto base_of = [&](uint32_t h) -> uint32_t {  // of the input tile
     if constexpr (LOW) {
-      base = (P.ladder ? h ^ (h >> 1) : h) << 12;
+      return (P.ladder ? h ^ (h >> 1) : h) << 12;
     } else {
       const int run = P.start - pas;  // free bits between the passengers and the targets
-      base = ((h & ((1u << run) - 1u)) << pas) | ((h >> run) << (P.start + cnt));
+      return ((h & ((1u << run) - 1u)) << pas) | ((h >> run) << (P.start + cnt));
     }
-    // consecutive chunks of a tile are consecutive in memory: chunk order over
-    // (passengers, targets), tile-local order (passengers 0-3, targets, other
-    // passengers)
-    auto local_of = [&](uint32_t i) -> uint32_t {
-      if constexpr (LOW) return i;
-      const uint32_t low = i & 15u, mid = (i >> 4) & ((1u << (pas - 4)) - 1u), tg = i >> pas;
-      return low | (tg << 4) | (mid << (4 + cnt));
-    };
-    auto global_of = [&](uint32_t i) -> uint32_t {
-      if constexpr (LOW) return base | i;
-      else return base | (i & ((1u << pas) - 1u)) | ((i >> pas) << P.start);
-    };
-    __syncthreads();  // the previous tile has left
+  };
+  auto load = [&](uint32_t t, float2* tile) {
+    const float2* src = P.src + ((size_t)(t >> (n - 12)) << n) + base_of(t & ((1u << (n - 12)) - 1u));
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const uint32_t i = 2 * tid + 512 * k;
-      cp_async<16>(smem_u32(tile + bslot(local_of(i))), P.src + state + global_of(i));
+      cp_async<16>(smem_u32(tile + bslot(local_of(i))), src + offset_of(i));
+    }
+    if ((int)tid < 4 * cnt) {
+      const double* m = P.mats + P.circ[t >> (n - 12)].mats_off + ((size_t)P.layer * n + (n - 1 - (P.start + (tid >> 2)))) * 8;
+      cp_async<16>(smem_u32(raw + tid), m + 2 * (tid & 3u));
     }
     cp_async_commit();
-    if (cid != have) {
-      have = cid;
-      if ((int)tid < 4 * cnt) {
-        const int j = tid >> 2;
-        const double* m = P.mats + P.circ[cid].mats_off + ((size_t)P.layer * n + (n - 1 - (P.start + j))) * 8;
-        const float x = (float)m[2 * (tid & 3u)], y = (float)m[2 * (tid & 3u) + 1];
-        um[(LOW ? 0 : 4) + j][tid & 3u] = make_float4(x, x, -y, y);
-      }
-    }
+  };
+  auto arrive = [&](int buf) {  // a thread converts the entry it has loaded itself
     cp_async_wait<0>();
-    __syncthreads();
+    if ((int)tid < 4 * cnt) {
+      const float x = (float)raw[tid].x, y = (float)raw[tid].y;
+      um[buf][(LOW ? 0 : 4) + (tid >> 2)][tid & 3u] = make_float4(x, x, -y, y);
+    }
+  };
+  int buf = 0;
+  if (blockIdx.x < P.n_tiles) {
+    load(blockIdx.x, tiles);
+    arrive(0);
+  }
+  for (uint32_t t = blockIdx.x; t < P.n_tiles; t += gridDim.x, buf ^= 1) {
+    // keeps the per-chunk addresses from being held (spilled) across tiles
+    asm volatile("" : "+r"(tid));
+    float2* tile = tiles + 4096 * buf;
+    __syncthreads();  // the tile and its matrices are here, the previous tile has left
+    const uint32_t next = t + gridDim.x;
+    if (next < P.n_tiles) load(next, tiles + 4096 * (buf ^ 1));
+    asm volatile("" : "+r"(tid));
     if constexpr (LOW) {
       if (cnt > 8) {
-        group_phase<2>(tile, tid, cnt - 8, &um[8]);
+        group_phase<2>(tile, tid, cnt - 8, &um[buf][8]);
         __syncthreads();
       }
       if (cnt > 4) {
-        group_phase<1>(tile, tid, min(cnt - 4, 4), &um[4]);
+        group_phase<1>(tile, tid, min(cnt - 4, 4), &um[buf][4]);
         __syncthreads();
       }
-      group_phase<0>(tile, tid, min(cnt, 4), &um[0]);
+      group_phase<0>(tile, tid, min(cnt, 4), &um[buf][0]);
     } else {
       if (cnt > 4) {
-        group_phase<2>(tile, tid, cnt - 4, &um[8]);
+        group_phase<2>(tile, tid, cnt - 4, &um[buf][8]);
         __syncthreads();
       }
-      group_phase<1>(tile, tid, min(cnt, 4), &um[4]);
+      group_phase<1>(tile, tid, min(cnt, 4), &um[buf][4]);
     }
     __syncthreads();
-    float2* out = P.dst + state;
+    asm volatile("" : "+r"(tid));
+    const uint32_t h = t & ((1u << (n - 12)) - 1u);
+    float2* out = P.dst + ((size_t)(t >> (n - 12)) << n) + (LOW ? h << 12 : base_of(h));
     const uint32_t cl = (h & 1u) << 11;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -307,11 +323,12 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_group_sweep(const
         uint32_t l = i;
         if (P.ladder) l = i ^ (i >> 1) ^ cl;
         const float4 v = *reinterpret_cast<const float4*>(tile + bslot(l & ~1u));
-        *reinterpret_cast<float4*>(out + ((h << 12) | i)) = (l & 1u) ? make_float4(v.z, v.w, v.x, v.y) : v;
+        *reinterpret_cast<float4*>(out + i) = (l & 1u) ? make_float4(v.z, v.w, v.x, v.y) : v;
       } else {
-        *reinterpret_cast<float4*>(out + global_of(i)) = *reinterpret_cast<const float4*>(tile + bslot(local_of(i)));
+        *reinterpret_cast<float4*>(out + offset_of(i)) = *reinterpret_cast<const float4*>(tile + bslot(local_of(i)));
       }
     }
+    if (next < P.n_tiles) arrive(buf ^ 1);
   }
 }
 
@@ -724,14 +741,14 @@ static int record_lane_groups(mq_batch* b, int l, float* probs, double* z0) {
       for (size_t g = 1; g < split.size(); ++g) {
         P.start = (uint8_t)split[g].first;
         P.cnt = (uint8_t)split[g].second;
-        k_group_sweep<false><<<grid(P.n_tiles), kSweepThreads, 0, s>>>(P);
+        k_group_sweep<false><<<grid(P.n_tiles), kSweepThreads, kSweepSmem, s>>>(P);
         MQ_LAUNCHED("k_group_sweep");
       }
       if (G.ladder) cur ^= 1;
       P.dst = buf[cur];
       P.start = 0;
       P.cnt = (uint8_t)split[0].second;
-      k_group_sweep<true><<<grid(P.n_tiles), kSweepThreads, 0, s>>>(P);
+      k_group_sweep<true><<<grid(P.n_tiles), kSweepThreads, kSweepSmem, s>>>(P);
       MQ_LAUNCHED("k_group_sweep");
     }
     GroupProbs Q;
@@ -949,6 +966,10 @@ int mq_batch_create(int device, void* stream, int n_circuits, const int32_t* n_q
     if (rc) { batch_free(b); return rc; }
   }
   if (!b->large.empty()) {
+    e = cudaFuncSetAttribute(k_group_sweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_group_sweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem);
+    if (e != cudaSuccess) return bail(e, "batch sweep setup");
     b->zblocks = (uint32_t)b->num_sms * 4;
     b->lanes = std::min<int>(lanes, (int)b->large.size());
     e = plan_groups(b);
