@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(NT) k_batch_small(const SmallCircuit* __restri
 // still that deep is one launch per sweep.  A sweep of one 14- to 20-qubit
 // circuit fills a fraction of the GPU for about 10 us, and a graph of one such
 // node per circuit, layer and sweep is bound by its nodes: 256 circuits of 10
-// to 20 qubits, 9.0 ms with 3400 sweeps of single circuits, 4.7 ms this way (20
+// to 20 qubits, 9.0 ms with 3400 sweeps of single circuits, 4.4 ms this way (20
 // qubits, 32 circuits: 5.2 -> 3.5 ms; 14 and 15 qubits, 100 circuits: 1.54 -> 0.42).
 // What bounds a sweep now is the complex 2x2 arithmetic and its latency (24 warps
 // an SM).  The gates of an amplitude are applied in the order and with the
@@ -189,8 +189,7 @@ constexpr size_t kSweepSmem = 2 * 4096 * sizeof(float2);
 // the first `cnt` of these bits in ascending order.  (Scalar FP32 instructions
 // instead of cmac2p: 5.19 against 4.98 ms a batch run.)
 template <int P>
-__device__ __forceinline__ void group_phase(float2* tile, uint32_t tid, int cnt, const float4 (*um)[4]) {
-  float2 a[16];
+__device__ __forceinline__ void group_gates(const float2* tile, uint32_t tid, int cnt, const float4 (*um)[4], float2 (&a)[16]) {
   if constexpr (P == 0) {
 #pragma unroll
     for (int r = 0; r < 16; r += 2) {
@@ -214,6 +213,11 @@ __device__ __forceinline__ void group_phase(float2* tile, uint32_t tid, int cnt,
       a[r | (1 << k)] = cmac2p(u[2], x0, u[3], x1);
     }
   }
+}
+template <int P>
+__device__ __forceinline__ void group_phase(float2* tile, uint32_t tid, int cnt, const float4 (*um)[4]) {
+  float2 a[16];
+  group_gates<P>(tile, tid, cnt, um, a);
   if constexpr (P == 0) {
 #pragma unroll
     for (int r = 0; r < 16; r += 2)
@@ -252,6 +256,10 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_group_sweep(const
   auto offset_of = [&](uint32_t i) -> uint32_t {
     if constexpr (LOW) return i;
     else return (i & ((1u << pas) - 1u)) | ((i >> pas) << P.start);
+  };
+  // high sweeps: offset of a tile-local index (bits 4 and up)
+  auto place = [&](uint32_t l) -> uint32_t {
+    return (((l >> 4) & ((1u << cnt) - 1u)) << P.start) | ((l >> (4 + cnt)) << 4);
   };
   auto base_of = [&](uint32_t h) -> uint32_t {  // of the input tile
     if constexpr (LOW) {
@@ -309,23 +317,33 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_group_sweep(const
         group_phase<2>(tile, tid, cnt - 4, &um[buf][8]);
         __syncthreads();
       }
-      group_phase<1>(tile, tid, min(cnt, 4), &um[buf][4]);
-    }
-    __syncthreads();
-    asm volatile("" : "+r"(tid));
-    const uint32_t h = t & ((1u << (n - 12)) - 1u);
-    float2* out = P.dst + ((size_t)(t >> (n - 12)) << n) + (LOW ? h << 12 : base_of(h));
-    const uint32_t cl = (h & 1u) << 11;
+      // the last phase's 16 amplitudes go straight to memory: 16 lanes are the
+      // passengers 0-3, so every run is a whole line (4.56 -> 4.42 ms a batch run)
+      float2 a[16];
+      group_gates<1>(tile, tid, min(cnt, 4), &um[buf][4], a);
+      asm volatile("" : "+r"(tid));
+      const uint32_t rest = (tid >> 4) << 8;  // tile bits 8-11
+      float2* out = P.dst + ((size_t)(t >> (n - 12)) << n) + base_of(t & ((1u << (n - 12)) - 1u)) + place(rest) + (tid & 15u);
+      uint32_t step[4];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t i = 2 * tid + 512 * k;
-      if constexpr (LOW) {
+      for (int k = 0; k < 4; ++k) step[k] = place(16u << k);
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        out[((r & 1) ? step[0] : 0u) + ((r & 2) ? step[1] : 0u) + ((r & 4) ? step[2] : 0u) + ((r & 8) ? step[3] : 0u)] = a[r];
+    }
+    if constexpr (LOW) {
+      __syncthreads();
+      asm volatile("" : "+r"(tid));
+      const uint32_t h = t & ((1u << (n - 12)) - 1u);
+      float2* out = P.dst + ((size_t)(t >> (n - 12)) << n) + (h << 12);
+      const uint32_t cl = (h & 1u) << 11;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t i = 2 * tid + 512 * k;
         uint32_t l = i;
         if (P.ladder) l = i ^ (i >> 1) ^ cl;
         const float4 v = *reinterpret_cast<const float4*>(tile + bslot(l & ~1u));
         *reinterpret_cast<float4*>(out + i) = (l & 1u) ? make_float4(v.z, v.w, v.x, v.y) : v;
-      } else {
-        *reinterpret_cast<float4*>(out + offset_of(i)) = *reinterpret_cast<const float4*>(tile + bslot(local_of(i)));
       }
     }
     if (next < P.n_tiles) arrive(buf ^ 1);

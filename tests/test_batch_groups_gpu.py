@@ -65,3 +65,23 @@ def test_groups_match_oracle(lanes):
                 assert abs(z0[c] - (ref[:half].sum() - ref[half:].sum())) < 1e-5 * total, (it, c, n, kinds[c])
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("n,count", [(14, 160), (16, 40)])
+def test_blocks_go_from_one_circuit_to_the_next(n, count):
+    """More tiles than resident blocks: a block's next tile belongs to another
+    circuit, whose matrices (and depth) differ."""
+    from mettleq_b200.batch import CircuitBatch
+    rng = np.random.default_rng(n)
+    ds = [2 + c % 3 for c in range(count)]
+    b = CircuitBatch([n] * count, ds, lanes=2)
+    try:
+        mats = [_mats("haar", d, n, rng) for d in ds]
+        b.run(mats)
+        for c in range(count):
+            p = _oracle(n, mats[c], True)
+            assert np.max(np.abs(b.probabilities(c) - p)) < 2e-6
+            z = p[: 1 << (n - 1)].sum() - p[1 << (n - 1):].sum()
+            assert abs(b.z0()[c] - z) < 1e-5
+    finally:
+        b.close()
