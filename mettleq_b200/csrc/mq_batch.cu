@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(NT) k_batch_small(const SmallCircuit* __restri
 // still that deep is one launch per sweep.  A sweep of one 14- to 20-qubit
 // circuit fills a fraction of the GPU for about 10 us, and a graph of one such
 // node per circuit, layer and sweep is bound by its nodes: 256 circuits of 10
-// to 20 qubits, 9.0 ms with 3400 sweeps of single circuits, 4.4 ms this way (20
+// to 20 qubits, 9.0 ms with 3400 sweeps of single circuits, 4.3 ms this way (20
 // qubits, 32 circuits: 5.2 -> 3.5 ms; 14 and 15 qubits, 100 circuits: 1.54 -> 0.42).
 // What bounds a sweep now is the complex 2x2 arithmetic and its latency (24 warps
 // an SM).  The gates of an amplitude are applied in the order and with the
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_group_sweep(const
       }
       if (cnt > 4) {
         group_phase<1>(tile, tid, min(cnt - 4, 4), &um[buf][4]);
-        __syncthreads();
+        __syncwarp();
       }
       group_phase<0>(tile, tid, min(cnt, 4), &um[buf][0]);
     } else {
@@ -332,14 +332,23 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_group_sweep(const
         out[((r & 1) ? step[0] : 0u) + ((r & 2) ? step[1] : 0u) + ((r & 4) ? step[2] : 0u) + ((r & 8) ? step[3] : 0u)] = a[r];
     }
     if constexpr (LOW) {
-      __syncthreads();
+      // phases 1 and 0 and the ladder keep tile bits 9-11 apart (the ladder
+      // maps each value to one), so a warp reads only what it wrote: two
+      // block barriers less, 4.42 -> 4.32 ms a batch run
+      __syncwarp();
       asm volatile("" : "+r"(tid));
       const uint32_t h = t & ((1u << (n - 12)) - 1u);
+      uint32_t block = tid >> 5;
+      if (P.ladder) {
+        block ^= (h & 1u) << 2;
+        block ^= block >> 1;
+        block ^= block >> 2;
+      }
       float2* out = P.dst + ((size_t)(t >> (n - 12)) << n) + (h << 12);
       const uint32_t cl = (h & 1u) << 11;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const uint32_t i = 2 * tid + 512 * k;
+        const uint32_t i = (block << 9) + 2 * (tid & 31u) + 64 * k;
         uint32_t l = i;
         if (P.ladder) l = i ^ (i >> 1) ^ cl;
         const float4 v = *reinterpret_cast<const float4*>(tile + bslot(l & ~1u));
