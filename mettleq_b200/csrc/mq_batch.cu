@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(NT) k_batch_small(const SmallCircuit* __restri
 // circuit fills a fraction of the GPU for about 10 us, and a graph of one such
 // node per circuit, layer and sweep is bound by its nodes: 256 circuits of 10
 // to 20 qubits, 9.0 ms with 3400 sweeps of single circuits, 4.3 ms this way (20
-// qubits, 32 circuits: 5.2 -> 3.5 ms; 14 and 15 qubits, 100 circuits: 1.54 -> 0.42).
+// qubits, 32 circuits: 5.2 -> 3.2 ms; 14 and 15 qubits, 100 circuits: 1.54 -> 0.42).
 // What bounds a sweep now is the complex 2x2 arithmetic and its latency (24 warps
 // an SM).  The gates of an amplitude are applied in the order and with the
 // rounding of the single circuits' sweeps (fill_order): the states are the same
