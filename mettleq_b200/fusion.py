@@ -346,7 +346,7 @@ _TERM_PARAMS = (1, 1, 1, 1, 1, 1, 4, 8)
 def _native_segments(operations: Sequence[dict], n: int) -> Optional[List[Dict[str, Any]]]:
     """The fused segments of ``fuse`` (before merging) from mq_fuse_stream, for
     streams of ordinary gates; None for any other stream (pseudo-ops, other
-    spellings of names, values that are not plain numbers, malformed gates),
+    spellings of names, values that are no finite numbers, malformed gates),
     which the Python rules below handle or refuse.  One pass over the op
     dicts builds the arrays; the per-gate work is native."""
     if not (1 <= n <= 31):
@@ -359,9 +359,12 @@ def _native_segments(operations: Sequence[dict], n: int) -> Optional[List[Dict[s
         n_wires = np.fromiter(map(len, wires), np.int32, count)
         n_params = np.fromiter(map(len, params), np.int32, count)
         flat_w = np.fromiter(chain.from_iterable(wires), np.int32, int(n_wires.sum()))
-        flat_p = np.fromiter(chain.from_iterable(params), np.float64, int(n_params.sum()))
+        # float() as the Python rules take it: numpy alone would turn None into NaN
+        flat_p = np.fromiter(map(float, chain.from_iterable(params)), np.float64, int(n_params.sum()))
         lib = N.lib()
     except (KeyError, TypeError, ValueError, OverflowError, AttributeError, RuntimeError):
+        return None
+    if not (np.abs(flat_p) < 1e300).all():  # infinities, NaN, and what sums to one
         return None
     code = np.array(codes, dtype=np.int32)
     ints = np.empty(3 * count * (n + 8) + 16, dtype=np.int32)

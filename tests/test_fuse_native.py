@@ -93,3 +93,31 @@ def test_an_iterator_of_gates_is_read_once(name):
 def test_malformed_gates_are_refused_as_before(op):
     with pytest.raises(ValueError):
         F.fuse([{"name": "H", "wires": [0], "parameters": []}, op], 3)
+
+
+def _outcome(fn):
+    try:
+        return fn()
+    except Exception as e:
+        return type(e)
+
+
+@pytest.mark.parametrize("value", [None, math.inf, -math.inf, math.nan, np.timedelta64(3, "s"), np.datetime64("2020-01-01"), "x",
+                                   1j, [0.5]])
+@pytest.mark.parametrize("name", ["RX", "U1", "U3", "CPHASE", "CRX", "XXPHASE", "ZZPHASE", "H"])
+def test_parameters_without_a_finite_value_follow_the_python_rules(name, value):
+    """An unbound (None) or non-finite parameter is refused, or carried along,
+    exactly as the Python rules do it: no gate becomes NaN unnoticed."""
+    count = max(1, F.PARAMS.get(name, 0))  # H: a parameter it does not use is still converted
+    ops = [{"name": name, "wires": list(range(F.ARITIES[name])), "parameters": [0.25] * (count - 1) + [value]}]
+    ref = _outcome(lambda: F._fuse_python(ops, 3, True))
+    got = _outcome(lambda: F.fuse(ops, 3))
+    if isinstance(ref, type):
+        assert got is ref
+        return
+    assert repr(got) == repr(ref)
+
+
+def test_angles_whose_sum_is_not_finite_are_refused():
+    with pytest.raises(ValueError):
+        F.fuse([{"name": "U3", "wires": [0], "parameters": [0.1, 1e308, 1e308]}], 3)
