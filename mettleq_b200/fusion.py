@@ -352,8 +352,8 @@ def _native_segments(operations: Sequence[dict], n: int) -> Optional[List[Dict[s
     if not (1 <= n <= 31):
         return None
     try:
-        codes = [_CODES[op["name"]] for op in operations]
-        wires = [op["wires"] for op in operations]
+        codes = [_CODES[op.get("name")] for op in operations]
+        wires = [op.get("wires", ()) for op in operations]
         params = [op.get("parameters") or () for op in operations]
         count = len(codes)
         n_wires = np.fromiter(map(len, wires), np.int32, count)

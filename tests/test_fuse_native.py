@@ -121,3 +121,13 @@ def test_parameters_without_a_finite_value_follow_the_python_rules(name, value):
 def test_angles_whose_sum_is_not_finite_are_refused():
     with pytest.raises(ValueError):
         F.fuse([{"name": "U3", "wires": [0], "parameters": [0.1, 1e308, 1e308]}], 3)
+
+
+def test_missing_keys_are_not_made_up():
+    """A gate without a name is refused even where the mapping has defaults,
+    and reading it adds no keys."""
+    from collections import defaultdict
+    op = defaultdict(lambda: "H", wires=[0])
+    with pytest.raises(ValueError):
+        F.fuse([op], 3)
+    assert set(op) == {"wires"}
