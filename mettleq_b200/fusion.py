@@ -362,7 +362,7 @@ def _native_segments(operations: Sequence[dict], n: int) -> Optional[List[Dict[s
         # float() as the Python rules take it: numpy alone would turn None into NaN
         flat_p = np.fromiter(map(float, chain.from_iterable(params)), np.float64, int(n_params.sum()))
         lib = N.lib()
-    except (KeyError, TypeError, ValueError, OverflowError, AttributeError, RuntimeError):
+    except (KeyError, TypeError, ValueError, OverflowError, AttributeError, RuntimeError, OSError):
         return None
     if not (np.abs(flat_p) < 1e300).all():  # infinities, NaN, and what sums to one
         return None

@@ -131,3 +131,13 @@ def test_missing_keys_are_not_made_up():
     with pytest.raises(ValueError):
         F.fuse([op], 3)
     assert set(op) == {"wires"}
+
+
+def test_a_library_that_does_not_load_leaves_the_python_rules(monkeypatch):
+    """Fusion is host code: it works where libmq.so or its CUDA runtime cannot
+    be loaded."""
+    def broken():
+        raise OSError("libcudart.so: cannot open shared object file")
+    monkeypatch.setattr(F.N, "lib", broken)
+    ops = [{"name": "H", "wires": [0], "parameters": []}]
+    assert F.fuse(ops, 2)[0]["active"] == [0]
