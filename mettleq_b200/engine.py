@@ -37,11 +37,13 @@ def _pack_terms(terms):
     k = len(terms)
     if k == 0:
         return None, None, None
-    kind, a, b, p = zip(*terms)
-    kinds = np.array(kind, dtype=np.int32)
+    kind, a, b, p = zip(*terms, strict=True)
+    # int() and list() entry by entry: what they take is what a term may hold
+    kinds = np.array(list(map(int, kind)), dtype=np.int32)
     wires = np.empty(2 * k, dtype=np.int32)
-    wires[0::2] = a
-    wires[1::2] = b
+    wires[0::2] = list(map(int, a))
+    wires[1::2] = list(map(int, b))
+    p = [list(x) for x in p]
     params = np.zeros((k, 8), dtype=np.float64)
     if all(len(x) == 1 for x in p):
         params[:, 0] = [x[0] for x in p]
