@@ -196,6 +196,8 @@ class AdjointEngine:
         self.ansatz, self.ham = ansatz, ham
         self.psi = StateVector(ansatz.n, dtype=dtype, device=device, stream=stream)
         self.lam = StateVector(ansatz.n, dtype=dtype, device=device, stream=self.psi.stream)
+        if not stream:  # psi's own stream ends with psi
+            self.psi._borrowers.append(self.lam)
         self._lib = N.lib()
         self._zm, self._zc, self._xc = ham.arrays()
 

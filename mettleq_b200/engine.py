@@ -156,10 +156,15 @@ class StateVector:
         self._lib = lib
         # host->device parameter bytes handed to kernels (end-to-end accounting)
         self.param_bytes = 0
+        # states on this handle's own stream: destroyed before it (close), since
+        # a destroy call waits for its stream
+        self._borrowers: List["StateVector"] = []
 
     # -- lifetime -------------------------------------------------------
     def close(self) -> None:
         if getattr(self, "_h", None) and self._h.value:
+            for sv in self._borrowers:
+                sv.close()
             self._lib.mq_state_destroy(self._h)
             self._h = C.c_void_p()
 
