@@ -29,6 +29,9 @@ int fail(int code, const std::string& msg) {
 
 int cuda_fail(cudaError_t e, const char* where) {
   const int code = (e == cudaErrorMemoryAllocation) ? MQ_ENOMEM : MQ_EDEVICE;
+  // reported here: not again by the check after the next call's launch (errors
+  // that end the context stay)
+  cudaGetLastError();
   return fail(code, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
