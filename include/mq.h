@@ -233,7 +233,10 @@ int mq_batch_run(mq_batch* b, const double* mats, float* probs_dev, double* z0_d
 /* The tile shape of the large circuits' sweeps (an autotuner's choice):
  * largest tile in bits (0 = default, else 6..12), low passenger bits of a
  * high sweep (-1 = default, else 0..5, fewer than tile_max), smallest tile
- * (0 = default).  Only before the first mq_batch_run. */
+ * (0 = default).  With any but the default plan (0, -1, 0) every circuit above
+ * 13 qubits runs on its own, not in groups of one width.  Only before the
+ * first mq_batch_run.  MQ_ENOMEM: the plan's device memory is not to be had,
+ * and the batch keeps the plan it had. */
 int mq_batch_set_tiles(mq_batch* b, int tile_max, int passengers, int tile_min);
 int mq_batch_sync(mq_batch* b);
 int mq_batch_destroy(mq_batch* b);

@@ -5,15 +5,16 @@ circuit (integrations/qiskit.py:505-514).  ``CircuitBatch`` hands a whole
 batch of layered circuits (per layer: a 2x2 on every qubit, then optionally
 the CNOT ladder) to ``mq_batch_*``: circuits of <= 13 qubits run whole in
 shared memory inside one persistent kernel, larger ones run tile sweeps on
-parallel streams, and the first run captures everything as one CUDA graph
+parallel streams (together with the others of their width up to 23 qubits, or
+one by one with a tile plan), and the first run captures everything as one CUDA graph
 that later runs replay with new parameters (the matrices are read from device
 memory).  Outputs stay on the device: every circuit's probability vector
 (float32) and <Z_0> (float64).
 
 ``autotune`` picks the batch's launch shape (threads per block of the
-shared-memory kernel, number of parallel lanes) and then the tile shape of
-the large circuits' sweeps (largest tile, passenger bits, smallest tile) by
-timing the candidates on the batch itself.
+shared-memory kernel, number of parallel lanes) and then how the large
+circuits run (the default plan, or one by one with a largest tile, passenger
+bits and a smallest tile) by timing the candidates on the batch itself.
 
 ``hea_batch`` generates the benchmark's batches: hardware-efficient ansatz
 circuits, RY and RZ angles U[-pi, pi] on every qubit per layer, then a CNOT
@@ -156,9 +157,10 @@ class CircuitBatch:
         return self.probs_dev[int(self.offsets[c]):int(self.offsets[c + 1])].cpu().numpy()
 
 
-# Tile shapes (largest tile, low passenger bits, smallest tile) the autotuner
-# tries for the large circuits: the library default first, then smaller and
-# larger tiles and fewer / more passengers (shorter / longer contiguous runs).
+# Plans (largest tile, low passenger bits, smallest tile) the autotuner tries for
+# the large circuits: the library default first (circuits of one width in
+# groups), then the circuits one by one with smaller and larger tiles and fewer
+# / more passengers (shorter / longer contiguous runs).
 TILE_CANDIDATES = ((0, -1, 0), (11, 4, 0), (10, 4, 0), (12, 3, 0), (12, 5, 0), (12, 4, 12))
 
 
@@ -185,9 +187,9 @@ def autotune(n_qubits: Sequence[int], depths: Sequence[int], packed: np.ndarray,
              cache: Optional[Dict] = None) -> Dict:
     """Choose the batch's launch shape and tile shape by timing them on this
     batch (graph capture excluded: each candidate runs once untimed):
-    first every (lanes, small_threads) pair with the default tiles, then
-    every tile shape of ``tiles`` (largest tile, passengers, smallest tile)
-    for the large circuits' sweeps with the best pair.  Returns the choice
+    first every (lanes, small_threads) pair with the default plan, then
+    every plan of ``tiles`` (largest tile, passengers, smallest tile; any but
+    the default runs the large circuits one by one) with the best pair.  Returns the choice
     with the time of every tile candidate.  ``cache`` (a dict) memoises the
     choice per batch signature."""
     key = (tuple(sorted(set(int(n) for n in n_qubits))), len(n_qubits), int(sum(depths)))

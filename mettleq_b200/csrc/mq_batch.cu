@@ -550,7 +550,7 @@ struct mq_batch {
   // large circuits
   std::vector<int> large;
   int lanes = 1;
-  std::vector<std::vector<int>> lane_work;  // single circuits (plan_singles)
+  std::vector<std::vector<int>> lane_work;  // single circuits (single_work)
   // groups of circuits of one width and ladder choice, deepest first
   struct Group {
     int n = 0;
@@ -560,6 +560,7 @@ struct mq_batch {
   };
   std::vector<Group> groups;
   std::vector<std::vector<int>> lane_groups;
+  std::vector<size_t> lane_amps;  // amplitudes of a lane's largest group
   std::vector<float2*> lane_buf[2];
   GroupCirc* d_group = nullptr;
   std::vector<cudaStream_t> lane_stream;
@@ -579,17 +580,18 @@ struct mq_batch {
 
 namespace mq {
 
+static void state_free(mq_state* h) {
+  if (h->buf[0]) cudaFree(h->buf[0]);
+  if (h->buf[1]) cudaFree(h->buf[1]);
+  if (h->scratch) cudaFree(h->scratch);
+  delete h;
+}
+
 static void batch_free(mq_batch* b) {
   if (!b) return;
   if (b->exec) cudaGraphExecDestroy(b->exec);
   for (auto& m : b->lane_state)
-    for (auto& kv : m) {
-      mq_state* h = kv.second;
-      if (h->buf[0]) cudaFree(h->buf[0]);
-      if (h->buf[1]) cudaFree(h->buf[1]);
-      if (h->scratch) cudaFree(h->scratch);
-      delete h;
-    }
+    for (auto& kv : m) state_free(kv.second);
   for (auto s : b->lane_stream) cudaStreamDestroy(s);
   for (auto e : b->lane_event) cudaEventDestroy(e);
   if (b->fork_event) cudaEventDestroy(b->fork_event);
@@ -607,9 +609,7 @@ static void batch_free(mq_batch* b) {
 
 // A lane's workspace state for n qubits (both buffers allocated up front:
 // nothing may allocate while the graph is being captured).
-static int lane_state_for(mq_batch* b, int lane, int n, mq_state** out) {
-  auto it = b->lane_state[lane].find(n);
-  if (it != b->lane_state[lane].end()) { *out = it->second; return MQ_OK; }
+static int make_lane_state(mq_batch* b, int lane, int n) {
   auto* h = new mq_state();
   h->n = n;
   h->dtype = MQ_C64;
@@ -624,12 +624,10 @@ static int lane_state_for(mq_batch* b, int lane, int n, mq_state** out) {
   cudaError_t e = cudaMalloc(&h->buf[0], h->state_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&h->buf[1], h->state_bytes);
   if (e != cudaSuccess) {
-    if (h->buf[0]) cudaFree(h->buf[0]);
-    delete h;
+    state_free(h);
     return cuda_fail(e, "cudaMalloc(batch lane state)");
   }
   b->lane_state[lane][n] = h;
-  *out = h;
   return MQ_OK;
 }
 
@@ -671,9 +669,7 @@ static int record_lane_single(mq_batch* b, int l, float* probs, double* z0) {
   double* zpart = b->d_zpart + (size_t)l * b->zslots;
   for (int c : b->lane_work[l]) {
     const int n = b->n[c];
-    mq_state* h = nullptr;
-    int rc = lane_state_for(b, l, n, &h);
-    if (rc) return rc;
+    mq_state* h = b->lane_state[l].at(n);
     h->cur = 0;
     MQ_CUDA(cudaMemsetAsync(h->buf[0], 0, h->state_bytes, s));
     k_basis0<<<1, 32, 0, s>>>(reinterpret_cast<float2*>(h->buf[0]));
@@ -682,7 +678,7 @@ static int record_lane_single(mq_batch* b, int l, float* probs, double* z0) {
     for (int j = 0; j < n; ++j) cols[j] = (1u << j) | (j ? (1u << (j - 1)) : 0u);
     for (int d = 0; d < b->depth[c]; ++d) {
       const double* md = b->d_mats + b->mats_off[c] + (size_t)d * n * 8;
-      rc = launch_layer(h, nullptr, nullptr, 0, nullptr, nullptr, nullptr, b->ladder[c] ? cols : nullptr, 0, md);
+      int rc = launch_layer(h, nullptr, nullptr, 0, nullptr, nullptr, nullptr, b->ladder[c] ? cols : nullptr, 0, md);
       if (rc) return rc;
     }
     const uint32_t dim = 1u << n;
@@ -795,7 +791,11 @@ static int record_lane_groups(mq_batch* b, int l, float* probs, double* z0) {
   return MQ_OK;
 }
 
-static bool single_circuits(const mq_batch* b) { return b->tile_max != 0 || b->tile_pas >= 0 || b->tile_min != 0; }
+// A tile plan other than the default: every large circuit runs on its own.
+static bool custom_tiles(int tile_max, int tile_pas, int tile_min) {
+  return tile_max != 0 || tile_pas >= 0 || tile_min != 0;
+}
+static bool single_circuits(const mq_batch* b) { return custom_tiles(b->tile_max, b->tile_pas, b->tile_min); }
 
 // Record the whole batch on b->stream (being captured).
 static int record_batch(mq_batch* b, float* probs, double* z0) {
@@ -828,37 +828,100 @@ constexpr size_t kGroupAmps = size_t(1) << 22;
 // The large circuits that run one by one, all of them with a tile plan set by
 // mq_batch_set_tiles, else those of 24 qubits and more, where the general
 // sweeps with TMA tiles are as fast (24 qubits, 6 circuits: 12.5 ms both; 23
-// qubits, 8 circuits: 8.6 against 8.2 ms in groups): their lanes (longest
-// processing time first) and the lanes' states, with the tile plan set so far.
+// qubits, 8 circuits: 8.6 against 8.2 ms in groups), by lane (longest
+// processing time first).
 constexpr int kGroupMaxQubits = 23;
-static int plan_singles(mq_batch* b) {
-  for (auto& m : b->lane_state)
-    for (auto& kv : m) {
-      kv.second->tile_max = b->tile_max;
-      kv.second->tile_pas = b->tile_pas;
-      kv.second->tile_min = b->tile_min;
-    }
-  b->lane_work.assign(b->lanes, {});
-  b->lane_state.resize(b->lanes);
+using LaneWork = std::vector<std::vector<int>>;
+static LaneWork single_work(const mq_batch* b, bool all) {
+  LaneWork work(b->lanes);
   std::vector<int> order;
   for (int c : b->large)
-    if (single_circuits(b) || b->n[c] > kGroupMaxQubits) order.push_back(c);
+    if (all || b->n[c] > kGroupMaxQubits) order.push_back(c);
   auto load = [&](int c) { return (uint64_t)std::max(1, b->depth[c]) << b->n[c]; };
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return load(x) > load(y); });
   std::vector<uint64_t> sum(b->lanes, 0);
   for (int c : order) {
     const int l = (int)(std::min_element(sum.begin(), sum.end()) - sum.begin());
-    b->lane_work[l].push_back(c);
+    work[l].push_back(c);
     sum[l] += load(c);
-    mq_state* h = nullptr;
-    int rc = lane_state_for(b, l, b->n[c], &h);
-    if (rc) return rc;
   }
+  return work;
+}
+
+// The device memory of a plan (its single circuits' states and, for the
+// default tiles, the groups' buffers): what is missing is allocated, what is
+// there stays.
+static int acquire(mq_batch* b, const LaneWork& work, bool groups) {
+  for (int i = 0; i < 2 && groups; ++i)
+    for (int l = 0; l < b->lanes; ++l) {
+      if (b->lane_buf[i][l] || !b->lane_amps[l]) continue;
+      const cudaError_t e = cudaMalloc(&b->lane_buf[i][l], b->lane_amps[l] * sizeof(float2));
+      if (e != cudaSuccess) {
+        b->lane_buf[i][l] = nullptr;
+        return cuda_fail(e, "cudaMalloc(batch group buffers)");
+      }
+    }
+  for (int l = 0; l < b->lanes; ++l)
+    for (int c : work[l])
+      if (!b->lane_state[l].count(b->n[c])) {
+        int rc = make_lane_state(b, l, b->n[c]);
+        if (rc) return rc;
+      }
+  return MQ_OK;
+}
+// Gives back what a plan does not use (nothing runs before the first capture).
+static void release_other(mq_batch* b, const LaneWork& work, bool groups) {
+  for (int l = 0; l < b->lanes; ++l) {
+    auto& m = b->lane_state[l];
+    for (auto it = m.begin(); it != m.end();) {
+      const bool used = std::any_of(work[l].begin(), work[l].end(), [&](int c) { return b->n[c] == it->first; });
+      if (used) {
+        ++it;
+      } else {
+        state_free(it->second);
+        it = m.erase(it);
+      }
+    }
+  }
+  for (int i = 0; i < 2 && !groups; ++i)
+    for (float2*& p : b->lane_buf[i]) {
+      if (p) cudaFree(p);
+      p = nullptr;
+    }
+}
+// Changes the tile plan as a whole or not at all: when the memory of the new
+// plan is not to be had, also not in place of the old plan's, the old plan is
+// in force again (mq_batch_run asks for its memory once more).
+static int change_plan(mq_batch* b, int tile_max, int tile_pas, int tile_min) {
+  const bool all = custom_tiles(tile_max, tile_pas, tile_min), had_all = single_circuits(b);
+  LaneWork work = single_work(b, all);
+  int rc = acquire(b, work, !all);
+  if (rc == MQ_ENOMEM) {
+    release_other(b, work, !all);
+    rc = acquire(b, work, !all);
+  }
+  if (rc) {
+    const std::string why = mq_last_error();
+    release_other(b, b->lane_work, !had_all);
+    acquire(b, b->lane_work, !had_all);
+    return fail(rc, why);
+  }
+  release_other(b, work, !all);
+  b->lane_work = std::move(work);
+  b->tile_max = tile_max;
+  b->tile_pas = tile_pas;
+  b->tile_min = tile_min;
+  for (auto& m : b->lane_state)
+    for (auto& kv : m) {
+      kv.second->tile_max = tile_max;
+      kv.second->tile_pas = tile_pas;
+      kv.second->tile_min = tile_min;
+    }
   return MQ_OK;
 }
 
 // Groups of the large circuits, their lanes (longest processing time first)
-// and device memory.
+// and their table (their buffers: acquire).
 static cudaError_t plan_groups(mq_batch* b) {
   std::map<std::pair<int, int>, std::vector<int>> by;  // (n, ladder)
   for (int c : b->large)
@@ -892,21 +955,17 @@ static cudaError_t plan_groups(mq_batch* b) {
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return load(b->groups[x]) > load(b->groups[y]); });
   std::vector<uint64_t> sum(b->lanes, 0);
-  std::vector<size_t> amps(b->lanes, 0);
+  b->lane_amps.assign(b->lanes, 0);
   for (int g : order) {
     const int l = (int)(std::min_element(sum.begin(), sum.end()) - sum.begin());
     b->lane_groups[l].push_back(g);
     sum[l] += load(b->groups[g]);
-    amps[l] = std::max(amps[l], b->groups[g].circ.size() << b->groups[g].n);
+    b->lane_amps[l] = std::max(b->lane_amps[l], b->groups[g].circ.size() << b->groups[g].n);
     b->zslots = std::max<size_t>(b->zslots, b->groups[g].circ.size() * group_blocks(b, b->groups[g].n));
   }
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < 2; ++i) {
-    b->lane_buf[i].assign(b->lanes, nullptr);
-    for (int l = 0; l < b->lanes && e == cudaSuccess; ++l)
-      if (amps[l]) e = cudaMalloc(&b->lane_buf[i][l], amps[l] * sizeof(float2));
-  }
-  if (e == cudaSuccess && !table.empty()) e = cudaMalloc(&b->d_group, table.size() * sizeof(GroupCirc));
+  for (auto& v : b->lane_buf) v.assign(b->lanes, nullptr);
+  if (!table.empty()) e = cudaMalloc(&b->d_group, table.size() * sizeof(GroupCirc));
   if (e == cudaSuccess && !table.empty())
     e = cudaMemcpy(b->d_group, table.data(), table.size() * sizeof(GroupCirc), cudaMemcpyHostToDevice);
   return e;
@@ -1013,10 +1072,10 @@ int mq_batch_create(int device, void* stream, int n_circuits, const int32_t* n_q
     }
     e = cudaEventCreateWithFlags(&b->fork_event, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(e, "cudaEventCreate(fork)");
-    {
-      int rc = plan_singles(b);
-      if (rc) { batch_free(b); return rc; }
-    }
+    b->lane_state.resize(b->lanes);
+    b->lane_work = single_work(b, false);
+    int rc = acquire(b, b->lane_work, true);
+    if (rc) { batch_free(b); return rc; }
     b->zslots = std::max<size_t>(b->zslots, b->zblocks);
     e = cudaMalloc(&b->d_zpart, (size_t)b->lanes * b->zslots * sizeof(double));
     if (e != cudaSuccess) return bail(e, "cudaMalloc(batch partials)");
@@ -1042,18 +1101,15 @@ int mq_batch_set_tiles(mq_batch* b, int tile_max, int passengers, int tile_min) 
   if (passengers < -1 || passengers > 5) return fail(MQ_EINVAL, "passengers must be -1 or in [0, 5]");
   if (tile_min < 0 || tile_min > 12) return fail(MQ_EINVAL, "tile_min must be 0 or in [1, 12]");
   if (tile_max && passengers >= tile_max) return fail(MQ_EINVAL, "passengers must leave room for targets in a tile");
-  b->tile_max = tile_max;
-  b->tile_pas = passengers;
-  b->tile_min = tile_min;
-  if (b->large.empty()) return MQ_OK;
+  if (b->large.empty()) {  // no sweeps: the plan is only noted
+    b->tile_max = tile_max;
+    b->tile_pas = passengers;
+    b->tile_min = tile_min;
+    return MQ_OK;
+  }
   MQ_TRY_BEGIN
   DeviceGuard g(b->device);
-  int rc = plan_singles(b);
-  if (rc) {
-    b->tile_max = b->tile_min = 0;
-    b->tile_pas = -1;
-  }
-  return rc;
+  return change_plan(b, tile_max, passengers, tile_min);
   MQ_TRY_END
 }
 
@@ -1069,6 +1125,10 @@ int mq_batch_run(mq_batch* b, const double* mats, float* probs_dev, double* z0_d
     if (b->exec) {
       cudaGraphExecDestroy(b->exec);
       b->exec = nullptr;
+    }
+    if (!b->large.empty()) {  // all there, unless a refused plan could not be undone
+      int rc = acquire(b, b->lane_work, !single_circuits(b));
+      if (rc) return rc;
     }
     MQ_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     int rc = record_batch(b, probs_dev, z0_dev);
