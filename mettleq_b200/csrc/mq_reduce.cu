@@ -16,6 +16,7 @@
 // offsets and a sequential running sum inside the chosen block.
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -307,6 +308,53 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint2 k) {
   return c;
 }
 
+// The target of shot s on the scale of the total.
+__device__ __forceinline__ double shot_target(int64_t s, uint64_t seed, uint64_t offset, double total) {
+  const uint64_t ctr = (uint64_t)s + offset;
+  const uint4 x = philox4x32_10(make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0u, 0u),
+                                make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
+  const uint64_t bits = ((((uint64_t)x.y) << 32) | x.x) >> 11;
+  const double u = (double)bits * 0x1p-53;
+  return __dmul_rn(u, total);
+}
+
+// One thread per shot: a binary search for the block, then its entries one
+// by one.  Bound by the latency of 1024 dependent reads and additions, about
+// 120 us whatever the number of shots, until they fill the GPU.  The better
+// one from kThreadShots shots: 20 qubits, a call of 16000 shots 232 us (170 with
+// a warp per shot), of 32000 262 (262), of 128000 572 (831); at 2 to 8 qubits
+// the two are equal near 16000.
+constexpr int64_t kThreadShots = 24576;
+template <typename Src>
+__global__ void k_draw_threads(Src src, uint32_t bs, uint32_t nb, const double* __restrict__ L,
+                               const double* __restrict__ E, const SampleMeta* __restrict__ meta, uint64_t seed,
+                               uint64_t offset, int64_t shots, int64_t* __restrict__ out) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= shots) return;
+  const double t = shot_target(s, seed, offset, meta->total);
+  uint32_t lo = 0, hi = nb - 1;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    const double c = __dadd_rn(E[mid / kSuper], L[mid]);
+    if (c <= t) lo = mid; else hi = mid - 1;
+  }
+  uint32_t b = lo;
+  if ((int32_t)b > meta->last_block) b = (uint32_t)max(meta->last_block, 0);
+  double r = __dadd_rn(E[b / kSuper], L[b]);
+  const uint32_t base = b * bs;
+  int64_t found = -1;
+  for (uint32_t i = 0; i < bs; ++i) {
+    r = __dadd_rn(r, src(base + i));
+    if (r > t) { found = i; break; }
+  }
+  if (found < 0) {
+    for (int64_t i = (int64_t)bs - 1; i >= 0; --i)
+      if (src(base + (uint32_t)i) > 0.0) { found = i; break; }
+    if (found < 0) found = 0;
+  }
+  out[s] = (int64_t)base + found;
+}
+
 // One warp per shot.  The block is found by a 32-way search over the
 // (non-decreasing) block offsets; its entries are staged in shared memory
 // with coalesced loads and summed in order by every lane alike (a broadcast
@@ -323,12 +371,7 @@ k_draw(Src src, uint32_t bs, uint32_t nb, const double* __restrict__ L, const do
   double* p = stage[warp];
   const int64_t s = (int64_t)blockIdx.x * kDrawWarps + warp;
   if (s >= shots) return;
-  const uint64_t ctr = (uint64_t)s + offset;
-  const uint4 x = philox4x32_10(make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0u, 0u),
-                                make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
-  const uint64_t bits = ((((uint64_t)x.y) << 32) | x.x) >> 11;
-  const double u = (double)bits * 0x1p-53;
-  const double t = __dmul_rn(u, meta->total);
+  const double t = shot_target(s, seed, offset, meta->total);
   // the last block whose offset is <= t (block 0 if none is)
   uint32_t lo = 0, hi = nb - 1;
   while (lo < hi) {
@@ -920,6 +963,11 @@ int run_probabilities(mq_state* h, const int32_t* wires, int k, int out_dtype, v
   return MQ_OK;
 }
 
+// Up to this many shots the call waits for the GPU once, and the shots pass
+// through host memory of its own; above, copying them twice takes longer than
+// the second wait.
+constexpr int64_t kStagedShots = 8192;
+
 template <typename Src>
 static int sample_from(mq_state* h, Src src, uint32_t m, uint64_t seed, uint64_t offset, int64_t shots,
                        int64_t* out, double* work) {
@@ -939,21 +987,41 @@ static int sample_from(mq_state* h, Src src, uint32_t m, uint64_t seed, uint64_t
   MQ_LAUNCHED("k_local_prefix");
   k_super_prefix<<<1, kPrefixThreads, 0, h->stream>>>(T, LP, ng, E, meta);
   MQ_LAUNCHED("k_super_prefix");
-  if (shots > 0) {
-    k_draw<Src><<<grid_for((uint64_t)shots, kDrawWarps), 32 * kDrawWarps, 0, h->stream>>>(src, bs, nb, L, E, meta, seed,
-                                                                                          offset, shots, dout);
-    MQ_LAUNCHED("k_draw");
-  }
-  // the total and the shots, which follow it, come back in one copy; a state
-  // without probability is refused then, before any shot is handed out
-  const size_t bytes = sizeof(SampleMeta) + (size_t)shots * 8;
-  std::vector<char> host(bytes);
-  MQ_CUDA(cudaMemcpyAsync(host.data(), meta, bytes, cudaMemcpyDeviceToHost, h->stream));
-  MQ_CUDA(cudaStreamSynchronize(h->stream));
   SampleMeta hm;
-  std::memcpy(&hm, host.data(), sizeof(hm));
-  if (!(hm.total > 0.0)) return fail(MQ_EINVAL, "Simulator returned a zero-probability state");
-  if (shots > 0) std::memcpy(out, host.data() + sizeof(SampleMeta), (size_t)shots * 8);
+  auto total = [&]() -> int {  // a state without probability is refused before any shot is handed out
+    if (!(hm.total > 0.0)) return fail(MQ_EINVAL, "Simulator returned a zero-probability state");
+    return MQ_OK;
+  };
+  if (shots <= kStagedShots) {
+    // the total and the shots, which follow it, come back in one copy
+    if (shots > 0) {
+      k_draw<Src><<<grid_for((uint64_t)shots, kDrawWarps), 32 * kDrawWarps, 0, h->stream>>>(
+          src, bs, nb, L, E, meta, seed, offset, shots, dout);
+      MQ_LAUNCHED("k_draw");
+    }
+    const size_t bytes = sizeof(SampleMeta) + (size_t)shots * 8;
+    std::unique_ptr<char[]> host(new char[bytes]);
+    MQ_CUDA(cudaMemcpyAsync(host.get(), meta, bytes, cudaMemcpyDeviceToHost, h->stream));
+    MQ_CUDA(cudaStreamSynchronize(h->stream));
+    std::memcpy(&hm, host.get(), sizeof(hm));
+    int rc = total();
+    if (rc) return rc;
+    if (shots > 0) std::memcpy(out, host.get() + sizeof(SampleMeta), (size_t)shots * 8);
+  } else {
+    MQ_CUDA(cudaMemcpyAsync(&hm, meta, sizeof(hm), cudaMemcpyDeviceToHost, h->stream));
+    MQ_CUDA(cudaStreamSynchronize(h->stream));
+    int rc = total();
+    if (rc) return rc;
+    if (shots < kThreadShots)
+      k_draw<Src><<<grid_for((uint64_t)shots, kDrawWarps), 32 * kDrawWarps, 0, h->stream>>>(
+          src, bs, nb, L, E, meta, seed, offset, shots, dout);
+    else
+      k_draw_threads<Src><<<grid_for((uint64_t)shots, 128), 128, 0, h->stream>>>(src, bs, nb, L, E, meta, seed, offset,
+                                                                                 shots, dout);
+    MQ_LAUNCHED("k_draw");
+    MQ_CUDA(cudaMemcpyAsync(out, dout, (size_t)shots * 8, cudaMemcpyDeviceToHost, h->stream));
+    MQ_CUDA(cudaStreamSynchronize(h->stream));
+  }
   h->launches += 4;
   h->sweeps += 1;
   return MQ_OK;
