@@ -6,12 +6,13 @@
 // apply_diagonal passes of the CPU path (sim.py:94-138, device.py:1154-1211).
 //
 // The reference multiplies one unit phase per equal-angle group inside the
-// kernel (zz.py:40-71); here the host factors the whole diagonal into at most
-// eight lookup tables, each indexed by a window of <= 10 index bits (or by a
-// short list of scattered bits for far-apart pairs).  Every term's phase is
-// folded into exactly one table in double precision, so a 29-bond chain with
-// all-different angles costs four table reads and four complex products per
-// amplitude, independent of the number of bonds.
+// kernel (zz.py:40-71).  Here a diagonal of unit-modulus terms is one angle per
+// amplitude, a quadratic form of its index bits, summed up by tiles (k_diag_tile,
+// below).  Small states and terms of other moduli take lookup tables (k_diag): the
+// host factors the whole diagonal into at most eight, each indexed by a window
+// of <= 10 index bits (or by a short list of scattered bits for far-apart pairs),
+// every term's phase folded into exactly one in double precision.  The fused
+// layers' epilogues use such tables too.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -139,6 +140,8 @@ struct Term {
   Few<int, 2> bits;                    // global index bits, first = MSB of table index
   Few<std::complex<double>, 4> tab;    // 2^|bits| values
   int lo = 0, hi = 0;                  // lowest and highest bit
+  int kind = 0;
+  double th = 0;                       // the angle of kinds that have one
 };
 
 struct PlannedLut {
@@ -166,6 +169,8 @@ static int build_terms(int n, int n_terms, const int32_t* kinds, const int32_t* 
     if (two && (b < 0 || b >= n || b == a)) return fail(MQ_EINVAL, "invalid bond (" + std::to_string(a) + ", " + std::to_string(b) + ")");
     Term tm;
     const double th = p[0];
+    tm.kind = kind;
+    tm.th = th;
     switch (kind) {
       case MQ_DIAG_ZZ: tm.tab = {cis(-th), cis(th), cis(th), cis(-th)}; break;
       case MQ_DIAG_CPHASE: tm.tab = {1.0, 1.0, 1.0, cis(th)}; break;
@@ -468,78 +473,140 @@ int plan_diag_register(mq_state* h, int n_terms, const int32_t* kinds, const int
 // The window tables above pay one look-up (for far bonds, one bit at a time)
 // and one complex product per table and amplitude, and a graph with many far
 // bonds needs eight of them.  This kernel uses that a term touches at most two
-// bits.  With t[b_a][b_b] = c u_a^{b_a} u_b^{b_b} w^{b_a b_b} the whole diagonal is
-//   c * prod_j u_j^{b_j} * prod_{i<j} w_ij^{b_i b_j},
+// bits: as an angle, the whole diagonal is
+//   c + sum_j u_j b_j + sum_{i<j} w_ij b_i b_j,
 // and for a tile of 2^M consecutive amplitudes (high bits H fixed) the pairs of
-// low bits are the same in every tile (a thread keeps its 16 or 8 factors in
-// shared memory), the pairs of high bits are one scalar, and the mixed pairs leave
-// one factor f_l = u_l prod_{h in H} w_lh per low bit.  One warp forms the f_l
-// and the scalar in float64 while the tile's loads are in flight, and 48
-// threads turn them into three tables over four bits, so an amplitude costs
-// three complex products whatever the graph.  Bound by memory: 26 qubits, a
-// ring and a random matching (38 bonds): 553 us with eight tables, 177 us
-// this way (6.1 TB/s).
+// low bits are the same in every tile (a thread keeps its 16 angles or 8 factors in
+// shared memory), the pairs of high bits are one angle, and the mixed pairs leave
+// one angle f_l = u_l + sum_{h in H} w_lh per low bit.  One warp adds up the f_l
+// while the tile's loads are in flight.  An amplitude's angle is then the sum of
+// three, whatever the graph: the thread's of the tile (eight bits), one of 16
+// over the other bits, and its static one; complex64 takes one sine and cosine of
+// the sum, complex128 (whose are long) multiplies three factors.
+// Angles are fixed-point fractions of a turn in 64 bits: their sums are exact,
+// whole turns drop out, and a factor is rounded once, where products of many
+// factors were off by up to twice as much as the tables (complex128, chain of
+// 17 qubits: 5.7e-16, the tables 3.2e-16, 1.5e-16 this way; complex64 6.7e-8,
+// 5.0e-8, 4.2e-8).
+// Bound by memory: 26 qubits, a chain and a random matching (38 bonds): 515 us
+// with eight tables, 173 us this way (6.2 TB/s); 12 qubits 3.8 and 3.7 us, 22
+// qubits 47 and 12 us.
 template <typename R> struct DiagTile;
 template <> struct DiagTile<float> { static constexpr int M = 12, CB = 1; };
 template <> struct DiagTile<double> { static constexpr int M = 11, CB = 0; };
 constexpr int kDiagLT = 8;  // 256 threads: index bits [CB, CB + 8)
-constexpr int kDiagCtas = 4;   // resident CTAs per SM: 64 registers a thread
+// resident CTAs per SM; 26 qubits, complex64: 192 us with one, 173 with two, 179
+// with three, 181 with four
+constexpr int kDiagCtas = 2;
 constexpr int kDiagHigh = 20;
+
+using Turn = unsigned long long;  // 2^-64 of a turn
 
 template <typename R>
 struct DiagTileParams {
   static constexpr int M = DiagTile<R>::M;
   uint32_t n_tiles;
   int32_t n;
-  double2 c;
-  double2 u[32];
-  double2 wl[M][M];            // w of low pairs (symmetric)
-  double2 wh[kDiagHigh][32];   // wh[h - M][j]: w of (j, h) for low j, and for high j with h < j (else 1)
+  Turn c;
+  Turn u[32];
+  Turn wl[M][M];            // w of low pairs (symmetric)
+  Turn wh[kDiagHigh][32];   // wh[h - M][j]: w of (j, h) for j < h (else 0)
 };
+
+// e^{i angle}: quarter turns exactly, the rest (at most an eighth of a turn) by
+// sincospi.
+__device__ __forceinline__ double2 turn_cis(Turn a) {
+  const unsigned q = (unsigned)((a + (Turn(1) << 61)) >> 62);
+  const double x = (double)(long long)(a - ((Turn)q << 62)) * 0x1p-63;
+  double s, c;
+  sincospi(x, &s, &c);
+  const double2 r = (q & 1u) ? make_double2(-s, c) : make_double2(c, s);
+  return (q & 2u) ? make_double2(-r.x, -r.y) : r;
+}
+
+// The same for two 32-bit angles (an error of 7e-10): the Taylor series of sine
+// and cosine on the rest, cut where the next term is below 2e-9, on the
+// paired FP32 instructions.  sincospif instead took 3 % longer at 26 qubits.
+__device__ __forceinline__ void turn_cis2(uint32_t a, uint32_t b, float2& x, float2& y) {
+  const uint32_t qa = (a + (1u << 29)) >> 30, qb = (b + (1u << 29)) >> 30;
+  const float2 r = make_float2((float)(int32_t)(a - (qa << 30)), (float)(int32_t)(b - (qb << 30)));
+  auto both = [](float v) { return make_float2(v, v); };
+  const float2 t = __fmul2_rn(r, both(1.4629180792671596e-9f));  // 2 pi / 2^32
+  const float2 u = __fmul2_rn(t, t);
+  float2 s = __ffma2_rn(u, both(1.f / 362880.f), both(-1.f / 5040.f));
+  s = __ffma2_rn(s, u, both(1.f / 120.f));
+  s = __ffma2_rn(s, u, both(-1.f / 6.f));
+  s = __ffma2_rn(__fmul2_rn(t, u), s, t);
+  float2 c = __ffma2_rn(u, both(-1.f / 3628800.f), both(1.f / 40320.f));
+  c = __ffma2_rn(c, u, both(-1.f / 720.f));
+  c = __ffma2_rn(c, u, both(1.f / 24.f));
+  c = __ffma2_rn(c, u, both(-0.5f));
+  c = __ffma2_rn(c, u, both(1.f));
+  auto turned = [](uint32_t q, float cs, float sn) {
+    const uint32_t sign = (q & 2u) << 30;
+    const float re = (q & 1u) ? -sn : cs, im = (q & 1u) ? cs : sn;
+    return make_float2(__uint_as_float(__float_as_uint(re) ^ sign), __uint_as_float(__float_as_uint(im) ^ sign));
+  };
+  x = turned(qa, c.x, s.x);
+  y = turned(qb, c.y, s.y);
+}
+__device__ __forceinline__ uint32_t turn_high(Turn a) { return (uint32_t)((a + (Turn(1) << 31)) >> 32); }
 
 template <typename R>
 __global__ void __launch_bounds__(1 << kDiagLT, kDiagCtas) k_diag_tile(V2<R>* __restrict__ st,
                                                             const __grid_constant__ DiagTileParams<R> P) {
   using T = V2<R>;
   constexpr int M = DiagTile<R>::M, CB = DiagTile<R>::CB;
+  constexpr bool C64 = sizeof(R) == 4;
   constexpr int NT = 1 << kDiagLT;
   constexpr int KB = M - kDiagLT;      // register bits: [0, CB) and [CB + 8, M)
   constexpr int NK = 1 << KB;
-  __shared__ double2 wh[kDiagHigh][32];
-  __shared__ double2 f[32];
-  __shared__ double2 scal;
-  __shared__ T tabA[16], tabB[16], tabK[16];
-  // a thread's static factors: two complex64 or one complex128 per 16 bytes
-  constexpr int SV = 1 << CB;
-  __shared__ __align__(16) T S[NK / SV][NT][SV];
+  __shared__ Turn wh[kDiagHigh][32];
+  __shared__ Turn f[32], scal;
+  __shared__ __align__(16) Turn ang[2][16];  // by four thread bits
+  // by register bits: complex64 angles, complex128 factors
+  __shared__ __align__(16) uint32_t angK[16];
+  __shared__ double2 tabK[C64 ? 1 : 16];
+  // a thread's static angles (four to 16 bytes) or factors
+  __shared__ uint4 S[C64 ? NK / 4 : NK][NT];
   const int tid = threadIdx.x;
   const int nh = P.n - M;
   for (int j = tid; j < nh * 32; j += NT) wh[j >> 5][j & 31] = P.wh[j >> 5][j & 31];
   auto reg_bit = [](int k) { return k < CB ? k : kDiagLT + k; };
-  // the static factors: pairs of low bits
+  // the static angles: pairs of low bits
   {
-    double2 base = make_double2(1.0, 0.0), cr[KB];
+    Turn base = 0, cr[KB];
 #pragma unroll
-    for (int k = 0; k < KB; ++k) cr[k] = make_double2(1.0, 0.0);
+    for (int k = 0; k < KB; ++k) cr[k] = 0;
+#pragma unroll 1
     for (int a = 0; a < kDiagLT; ++a) {
-      if (!((tid >> a) & 1)) continue;
-      for (int b = 0; b < a; ++b)
-        if ((tid >> b) & 1) base = cmul(base, P.wl[CB + a][CB + b]);
+      const Turn on = (tid >> a) & 1 ? ~Turn(0) : 0;
+      Turn with = 0;
 #pragma unroll
-      for (int k = 0; k < KB; ++k) cr[k] = cmul(cr[k], P.wl[CB + a][reg_bit(k)]);
+      for (int b = 0; b < kDiagLT; ++b)
+        if (b < a && ((tid >> b) & 1)) with += P.wl[CB + a][CB + b];
+      base += with & on;
+#pragma unroll
+      for (int k = 0; k < KB; ++k) cr[k] += P.wl[CB + a][reg_bit(k)] & on;
     }
+    uint32_t w[4];
 #pragma unroll
     for (int x = 0; x < NK; ++x) {
-      double2 v = base;
+      Turn v = base;
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
         if (!((x >> k) & 1)) continue;
-        v = cmul(v, cr[k]);
+        v += cr[k];
 #pragma unroll
         for (int i = 0; i < k; ++i)
-          if ((x >> i) & 1) v = cmul(v, P.wl[reg_bit(k)][reg_bit(i)]);
+          if ((x >> i) & 1) v += P.wl[reg_bit(k)][reg_bit(i)];
       }
-      S[x / SV][tid][x % SV] = mk<R>((R)v.x, (R)v.y);
+      if constexpr (C64) {
+        w[x & 3] = turn_high(v);
+        if ((x & 3) == 3) S[x / 4][tid] = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+        *reinterpret_cast<double2*>(&S[x][tid]) = turn_cis(v);
+      }
     }
   }
   __syncthreads();
@@ -548,7 +615,7 @@ __global__ void __launch_bounds__(1 << kDiagLT, kDiagCtas) k_diag_tile(V2<R>* __
     T a[NK];
 #pragma unroll
     for (int k = 0; k < (NK >> CB); ++k) {
-      if constexpr (CB == 1) {
+      if constexpr (C64) {
         const float4 v = reinterpret_cast<const float4*>(at)[tid + k * NT];
         a[2 * k] = mk<R>(v.x, v.y);
         a[2 * k + 1] = mk<R>(v.z, v.w);
@@ -558,38 +625,51 @@ __global__ void __launch_bounds__(1 << kDiagLT, kDiagCtas) k_diag_tile(V2<R>* __
     }
     if (tid < 32) {
       const int j = tid;
-      double2 g = j < P.n ? P.u[j] : make_double2(1.0, 0.0);
+      Turn g = j < P.n ? P.u[j] : 0;
       for (int h = 0; h < nh; ++h)
-        if ((t >> h) & 1u) g = cmul(g, wh[h][j]);
+        if ((t >> h) & 1u) g += wh[h][j];
       f[j] = g;
-      // the scalar: the product over the set high bits
-      double2 v = (j >= M && j < P.n && ((t >> (j - M)) & 1u)) ? g : make_double2(1.0, 0.0);
+      // the pairs of high bits and the set high bits' own angles
+      Turn v = (j >= M && j < P.n && ((t >> (j - M)) & 1u)) ? g : 0;
 #pragma unroll
-      for (int off = 16; off; off >>= 1)
-        v = cmul(v, make_double2(__shfl_xor_sync(0xffffffffu, v.x, off), __shfl_xor_sync(0xffffffffu, v.y, off)));
-      if (j == 0) scal = cmul(v, P.c);
+      for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+      if (j == 0) scal = v + P.c;
     }
     __syncthreads();
     if (tid < 48) {
       const int which = tid >> 4, x = tid & 15;
-      double2 v = which == 2 ? scal : make_double2(1.0, 0.0);
+      Turn v = which == 2 ? scal : 0;
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (((x >> k) & 1) && (which < 2 || k < KB)) v = cmul(v, f[which == 2 ? reg_bit(k) : CB + 4 * which + k]);
-      (which == 0 ? tabA : which == 1 ? tabB : tabK)[x] = mk<R>((R)v.x, (R)v.y);
+        if (((x >> k) & 1) && (which < 2 || k < KB)) v += f[which == 2 ? reg_bit(k) : CB + 4 * which + k];
+      if (which < 2) ang[which][x] = v;
+      else if constexpr (C64) angK[x] = turn_high(v);
+      else tabK[x] = turn_cis(v);
     }
     __syncthreads();
-    const T p = cmul(tabA[tid & 15], tabB[tid >> 4]);
+    const Turn mine = ang[0][tid & 15] + ang[1][tid >> 4];
+    if constexpr (C64) {
+      const uint32_t p = turn_high(mine);
 #pragma unroll
-    for (int x = 0; x < NK; x += SV) {
-      const float4 sv = *reinterpret_cast<const float4*>(&S[x / SV][tid][0]);
-      const T* s = reinterpret_cast<const T*>(&sv);
+      for (int x = 0; x < NK; x += 4) {
+        const uint4 s = S[x / 4][tid], k = *reinterpret_cast<const uint4*>(angK + x);
+        T w[4];
+        turn_cis2(p + k.x + s.x, p + k.y + s.y, w[0], w[1]);
+        turn_cis2(p + k.z + s.z, p + k.w + s.w, w[2], w[3]);
 #pragma unroll
-      for (int i = 0; i < SV; ++i) a[x + i] = cmul(a[x + i], cmul(s[i], cmul(p, tabK[x + i])));
+        for (int i = 0; i < 4; ++i) a[x + i] = cmul(a[x + i], w[i]);
+      }
+    } else {
+      const double2 p = turn_cis(mine);
+#pragma unroll
+      for (int x = 0; x < NK; ++x) {
+        const double2 s = *reinterpret_cast<const double2*>(&S[x][tid]);
+        a[x] = cmul(a[x], cmul(s, cmul(p, tabK[x])));
+      }
     }
 #pragma unroll
     for (int k = 0; k < (NK >> CB); ++k) {
-      if constexpr (CB == 1)
+      if constexpr (C64)
         reinterpret_cast<float4*>(at)[tid + k * NT] = make_float4(a[2 * k].x, a[2 * k].y, a[2 * k + 1].x, a[2 * k + 1].y);
       else
         at[tid + k * NT] = a[k];
@@ -597,39 +677,74 @@ __global__ void __launch_bounds__(1 << kDiagLT, kDiagCtas) k_diag_tile(V2<R>* __
   }
 }
 
+// Angles to 2^-62 of a turn: of x turns, |x| <= 1/2; of a number of modulus 1.
+static Turn to_turn(long double x) { return (Turn)std::llrint(x * 0x1p62L) << 2; }
+constexpr long double kPerTurn = 0.159154943091895335768883763372514362L;  // 1 / (2 pi)
+static Turn turn_of(std::complex<double> z) {
+  return z == 1.0 ? 0 : to_turn(std::atan2((long double)z.imag(), (long double)z.real()) * kPerTurn);
+}
+// The angles of a term's table entries: from its own angle where it has one
+// (an arctangent a term takes longer than the rest of the plan), and small
+// enough for the product to keep 2^-62 of a turn.
+static void term_turns(const Term& t, Turn (&a)[4]) {
+  const bool has = t.kind != MQ_DIAG_1Q && t.kind != MQ_DIAG_2Q && std::fabs(t.th) <= 8.0;
+  if (!has) {
+    for (size_t i = 0; i < t.tab.size(); ++i) {
+      size_t k = 0;  // equal and conjugate entries share one
+      while (k < i && t.tab[k] != t.tab[i] && t.tab[k] != std::conj(t.tab[i])) ++k;
+      a[i] = k == i ? turn_of(t.tab[i]) : t.tab[k] == t.tab[i] ? a[k] : 0 - a[k];
+    }
+    return;
+  }
+  const bool half = t.kind == MQ_DIAG_CRZ || t.kind == MQ_DIAG_RZ;
+  long double x = (long double)(half ? t.th / 2 : t.th) * kPerTurn;
+  const Turn w = t.tab[t.tab.size() - 1] == -1.0 ? Turn(1) << 63 : to_turn(x - std::rint(x));
+  switch (t.kind) {
+    case MQ_DIAG_ZZ: a[0] = a[3] = 0 - w; a[1] = a[2] = w; break;
+    case MQ_DIAG_CPHASE: a[0] = a[1] = a[2] = 0; a[3] = w; break;
+    case MQ_DIAG_CRZ: a[0] = a[1] = 0; a[2] = 0 - w; a[3] = w; break;
+    case MQ_DIAG_RZ: a[0] = 0 - w; a[1] = w; break;
+    default: a[0] = 0; a[1] = w; break;  // MQ_DIAG_PHASE
+  }
+}
+
 // The tiled form of a diagonal, when it has one: every table entry of modulus 1
-// (the factored form divides by them) and at least one whole tile.
+// to the rounding of its parts (complex64: to a hundredth of a result's), as
+// an angle keeps no modulus, and at least one whole tile.
 template <typename R>
 static bool plan_diag_tile(int n, const std::vector<Term>& terms, std::complex<double> scalar, DiagTileParams<R>& P) {
   constexpr int M = DiagTile<R>::M;
+  constexpr double off = sizeof(R) == 4 ? 1e-9 : 4.5e-16;
   if (n < M || n - M > kDiagHigh) return false;
-  std::vector<std::complex<double>> u(n, 1.0), w((size_t)n * n, 1.0);
-  for (const Term& t : terms) {
+  for (const Term& t : terms)
     for (const auto& v : t.tab)
-      if (!(std::fabs(std::abs(v) - 1.0) < 1e-6)) return false;
-    scalar *= t.tab[0];
-    if (t.bits.size() == 1) {
-      u[t.bits[0]] *= t.tab[1] / t.tab[0];
-      continue;
-    }
-    const int a = t.bits[0], b = t.bits[1];  // table index = 2 b_a + b_b
-    u[a] *= t.tab[2] / t.tab[0];
-    u[b] *= t.tab[1] / t.tab[0];
-    const auto v = t.tab[3] * t.tab[0] / (t.tab[1] * t.tab[2]);
-    w[(size_t)a * n + b] *= v;
-    w[(size_t)b * n + a] *= v;
-  }
-  auto d2 = [](std::complex<double> v) { return make_double2(v.real(), v.imag()); };
+      if (!(std::fabs(std::norm(v) - 1.0) <= off)) return false;
+  if (!(std::fabs(std::norm(scalar) - 1.0) <= 16 * off)) return false;
   std::memset(&P, 0, sizeof(P));
   P.n = n;
   P.n_tiles = 1u << (n - M);
-  P.c = d2(scalar);
-  for (int j = 0; j < n; ++j) P.u[j] = d2(u[j]);
-  for (int a = 0; a < M; ++a)
-    for (int b = 0; b < M; ++b) P.wl[a][b] = d2(w[(size_t)a * n + b]);
-  for (int h = M; h < n; ++h)
-    for (int j = 0; j < 32; ++j)
-      P.wh[h - M][j] = (j < M || (h < j && j < n)) ? d2(w[(size_t)j * n + h]) : make_double2(1.0, 0.0);
+  P.c = turn_of(scalar);
+  auto pair = [&](int h, int l, Turn w) {  // h > l
+    if (h >= M) {
+      P.wh[h - M][l] += w;
+    } else {
+      P.wl[h][l] += w;
+      P.wl[l][h] += w;
+    }
+  };
+  for (const Term& t : terms) {
+    Turn a[4];
+    term_turns(t, a);
+    P.c += a[0];
+    if (t.bits.size() == 1) {
+      P.u[t.bits[0]] += a[1] - a[0];
+      continue;
+    }
+    const int x = t.bits[0], y = t.bits[1];  // table index = 2 b_x + b_y
+    P.u[x] += a[2] - a[0];
+    P.u[y] += a[1] - a[0];
+    pair(t.hi, t.lo, a[3] - a[1] - a[2] + a[0]);
+  }
   return true;
 }
 
@@ -649,11 +764,6 @@ int launch_diag_terms(mq_state* h, int n_terms, const int32_t* kinds, const int3
   int rc = build_terms(h->n, n_terms, kinds, wires, params, terms, scalar);
   if (rc) return rc;
   if (terms.empty() && scalar == std::complex<double>(1.0, 0.0)) return MQ_OK;
-  // The tiled form wherever it exists.  It measured faster than the window
-  // tables for chains too (26 qubits: 177 against 219 us; complex128, 25
-  // qubits: 176 against 201 us), at 18 qubits and more on the device alone
-  // (6.2 against 9.6 us) and below that because the host plans no windows (12
-  // qubits: 39 against 63 us a call, of which 5.5 against 3.6 us on the device).
   if (h->dtype == MQ_C64) {
     DiagTileParams<float> P;
     if (plan_diag_tile(h->n, terms, scalar, P)) return launch_diag_tile(h, P);
