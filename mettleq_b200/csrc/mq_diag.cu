@@ -8,11 +8,11 @@
 // The reference multiplies one unit phase per equal-angle group inside the
 // kernel (zz.py:40-71).  Here a diagonal of unit-modulus terms is one angle per
 // amplitude, a quadratic form of its index bits, summed up by tiles (k_diag_tile,
-// below).  Small states and terms of other moduli take lookup tables (k_diag): the
-// host factors the whole diagonal into at most eight, each indexed by a window
-// of <= 10 index bits (or by a short list of scattered bits for far-apart pairs),
-// every term's phase folded into exactly one in double precision.  The fused
-// layers' epilogues use such tables too.
+// below).  Small states, diagonals that are one small table and terms of other
+// moduli take lookup tables (k_diag): the host factors the whole diagonal into
+// at most eight, each indexed by a window of <= 10 index bits (or by a short list
+// of scattered bits for far-apart pairs), every term's phase folded into exactly
+// one in double precision.  The fused layers' epilogues use such tables too.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -758,18 +758,43 @@ static int launch_diag_tile(mq_state* h, const DiagTileParams<R>& P) {
   return MQ_OK;
 }
 
+// Diagonals that are one small table stay with it: a look-up costs less than the
+// tile's angles.  Measured, us on the device, table against tile (complex64):
+// terms within six neighbouring bits, 14 qubits 1.7 / 3.8, 20 qubits 3.4 / 6.3,
+// 22 qubits 7.4 / 12.1, 24 qubits 45.4 / 45.6, 26 qubits 174 / 173; up to four
+// bits in pairs ten and more apart, 20 qubits 4.8 / 6.3, 22 qubits 13.6 / 12.1, 24
+// qubits 56 / 46.  complex128: 20 qubits 5.8 and 6.3 / 9.7, 22 qubits 21.2 and 18.1 /
+// 20.4, 24 qubits 97 / 90.  With more tables the tile is faster from 14 qubits on,
+// and below as a call (12 qubits, chain: 53 against 62 us, of which 3.7 against
+// 3.4 on the device: the host fills no tables).
+static bool one_small_table(int n, int dtype, const std::vector<Term>& terms) {
+  int lo = n, hi = -1;
+  bool apart = true;
+  uint32_t bits = 0;
+  for (const Term& t : terms) {
+    lo = std::min(lo, t.lo);
+    hi = std::max(hi, t.hi);
+    apart = apart && t.hi - t.lo >= 10;
+    for (int b : t.bits) bits |= 1u << b;
+  }
+  if (hi - lo < 6) return dtype == MQ_C64 || n <= 23;
+  return apart && __builtin_popcount(bits) <= 4 && n <= (dtype == MQ_C64 ? 21 : 23);
+}
+
 int launch_diag_terms(mq_state* h, int n_terms, const int32_t* kinds, const int32_t* wires, const double* params) {
   std::vector<Term> terms;
   std::complex<double> scalar;
   int rc = build_terms(h->n, n_terms, kinds, wires, params, terms, scalar);
   if (rc) return rc;
   if (terms.empty() && scalar == std::complex<double>(1.0, 0.0)) return MQ_OK;
-  if (h->dtype == MQ_C64) {
-    DiagTileParams<float> P;
-    if (plan_diag_tile(h->n, terms, scalar, P)) return launch_diag_tile(h, P);
-  } else {
-    DiagTileParams<double> P;
-    if (plan_diag_tile(h->n, terms, scalar, P)) return launch_diag_tile(h, P);
+  if (!one_small_table(h->n, h->dtype, terms)) {
+    if (h->dtype == MQ_C64) {
+      DiagTileParams<float> P;
+      if (plan_diag_tile(h->n, terms, scalar, P)) return launch_diag_tile(h, P);
+    } else {
+      DiagTileParams<double> P;
+      if (plan_diag_tile(h->n, terms, scalar, P)) return launch_diag_tile(h, P);
+    }
   }
   const int cap = h->dtype == MQ_C64 ? DiagCap<float>::v : DiagCap<double>::v;
   std::vector<PlannedLut> luts;

@@ -1,10 +1,12 @@
-"""Diagonals as sums of angles: accuracy and exact signs."""
+"""Diagonals as sums of angles: accuracy, exact signs, and the diagonals that
+are one small table."""
 import math
 
 import numpy as np
 import pytest
 
-from tests.helpers import rand_state
+from oracle import OracleSim
+from tests.helpers import oracle_apply_terms, rand_state
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +66,24 @@ def test_quarter_turns_are_exact(dtype):
         quarter += {1: 2 * x * ((i >> (n - 1 - b)) & 1), 3: 2 * x, 6: x}[kind]
     ref = np.choose(quarter % 4, [vec, -vec.imag + 1j * vec.real, -vec, vec.imag - 1j * vec.real]).astype(dtype)
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+@pytest.mark.parametrize("n", [11, 12, 13, 17, 22, 23, 24])
+def test_small_tables_and_tiles_agree_with_the_oracle(n, dtype):
+    """On both sides of the rule for one small table: spans of six and seven
+    bits, up to four and five scattered bits, a global phase alone."""
+    rng = np.random.default_rng(n)
+    t = lambda: [float(rng.uniform(-3, 3))]
+    sets = [[(2, n // 2, -1, t())], [(0, q, q + 1, t()) for q in range(2, 7)], [(0, q, q + 1, t()) for q in range(2, 8)],
+            [(5, 0, -1, t())]]
+    if n >= 14:
+        sets += [[(0, 0, n - 1, t()), (1, 1, n - 1, t()), (4, n - 2, 0, t())], [(0, 0, n - 1, t()), (0, 1, n - 2, t()), (0, 2, n - 1, t())]]
+    if n > 17:
+        sets = [sets[i] for i in (1, 4)]
+    vec = rand_state(n, n, dtype)
+    for terms in sets:
+        o = OracleSim(n, np.complex128)
+        o.set_state(vec.astype(np.complex128))
+        oracle_apply_terms(o, terms)
+        assert np.max(np.abs(_apply(n, dtype, vec, terms) - o.state)) <= (1e-6 if dtype == np.complex64 else 1e-14)
