@@ -37,6 +37,17 @@ def _pack_terms(terms):
     k = len(terms)
     if k == 0:
         return None, None, None
+    if k < 8:  # entry by entry: 1.7 to 6 us, by columns 3.7 to 6.7 (20 terms 15 and 11)
+        kinds = np.empty(k, dtype=np.int32)
+        wires = np.empty(2 * k, dtype=np.int32)
+        params = np.zeros((k, 8), dtype=np.float64)
+        for i, (kind, a, b, p) in enumerate(terms):
+            kinds[i] = int(kind)
+            wires[2 * i] = int(a)
+            wires[2 * i + 1] = int(b)
+            pp = list(p)
+            params[i, :len(pp)] = pp
+        return kinds, wires, params
     kind, a, b, p = zip(*terms, strict=True)
     # int() and list() entry by entry: what they take is what a term may hold
     kinds = np.array(list(map(int, kind)), dtype=np.int32)

@@ -30,6 +30,25 @@ def test_terms_are_accepted_as_written(make):
         assert got.dtype == ref.dtype and np.array_equal(got, ref)
 
 
+_MANY = [(0, q, q + 1, [0.1 * q]) for q in range(9)]
+
+
+@pytest.mark.parametrize("extra", [[], [(0, 0, 1, iter([0.3]))], [("1", 2.0, np.int64(3), (0.5,))], [(6, 0, -1, [1, 0, 0, 1])],
+                                   [(0, 1, 2, {0.4})]])
+def test_longer_lists_of_terms(extra):
+    """The same by columns; an iterator among the parameters is read once."""
+    ref = _plain(_MANY + [(k, a, b, [0.3]) if hasattr(p, "__next__") else (k, a, b, p) for k, a, b, p in extra])
+    for got, want in zip(_pack_terms(_MANY + extra), ref):
+        assert got.dtype == want.dtype and np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("bad", [(0, 1, 2, [0.4], 9), (0, 1, 2), (0, None, 1, [0.1]), (0, [1], 1, [0.1]), (0, 1, 2, 0.3),
+                                 (0, float("nan"), 1, [0.1])])
+def test_longer_lists_with_a_malformed_term(bad):
+    with pytest.raises((TypeError, ValueError)):
+        _pack_terms(_MANY + [bad])
+
+
 @pytest.mark.parametrize("make", [
     lambda: [(0, 0, 1, [0.3]), (0, 1, 2, [0.4], 9)],
     lambda: [(0, 0, 1, [0.3]), (0, 1, 2)],
