@@ -200,6 +200,7 @@ int mq_adjoint_layer_xor_async(mq_state* psi, mq_state* lam, const uint64_t* row
  * FREDKIN), n_wires[i] entries of wires and n_params[i] of params (each list
  * flat, in order).  Writes the fused segments to ints / doubles; used[0] and
  * used[1] are the entries written (MQ_EUNSUPPORTED when a capacity is less).
+ * MQ_EINVAL: a malformed gate, or a parameter of 1e300 or more or no number.
  * A segment of ints is one of
  *   0 j m inverse                       QFT stage j of the wires [j, m)
  *   1 k q[k]                            2x2 matrices (8 doubles each)

@@ -321,6 +321,7 @@ int mq_fuse_stream(int n, int n_ops, const int32_t* codes, const int32_t* n_wire
       if (g < 0 || g >= G_COUNT) return fail(MQ_EINVAL, "unknown gate code");
       if (n_wires[i] != arity(g)) return fail(MQ_EINVAL, "wrong wire count");
       if (n_params[i] < kParams[g]) return fail(MQ_EINVAL, "too few parameters");
+      if (n_params[i] > 0 && !params) return fail(MQ_EINVAL, "null stream arrays");
       Op o{};
       o.code = g;
       for (int k = 0; k < arity(g); ++k) {
@@ -329,6 +330,9 @@ int mq_fuse_stream(int n, int n_ops, const int32_t* codes, const int32_t* n_wire
         for (int l = 0; l < k; ++l)
           if (o.w[l] == o.w[k]) return fail(MQ_EINVAL, "Control/target wires must be distinct");
       }
+      // (infinities, NaN, and angles whose sum could be one: 1e300)
+      for (int k = 0; k < n_params[i]; ++k)
+        if (!(std::fabs(params[pi + k]) < 1e300)) return fail(MQ_EINVAL, "parameter is not finite");
       for (int k = 0; k < kParams[g]; ++k) o.p[k] = params[pi + k];
       wi += n_wires[i];
       pi += n_params[i];

@@ -141,3 +141,30 @@ def test_a_library_that_does_not_load_leaves_the_python_rules(monkeypatch):
     monkeypatch.setattr(F.N, "lib", broken)
     ops = [{"name": "H", "wires": [0], "parameters": []}]
     assert F.fuse(ops, 2)[0]["active"] == [0]
+
+
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan, 1e300])
+def test_the_c_entry_refuses_parameters_that_are_not_finite(value):
+    import ctypes as C
+    from mettleq_b200 import _native as N
+    i32 = C.c_int32 * 1
+    out, used = (C.c_int32 * 64)(), (C.c_int64 * 2)()
+    for code in (F.GATE_NAMES.index("RX"), F.GATE_NAMES.index("H")):  # H: a parameter it does not use
+        rc = N.lib().mq_fuse_stream(2, 1, i32(code), i32(1), i32(0), i32(1), (C.c_double * 1)(value), out, 64,
+                                    (C.c_double * 64)(), 64, used)
+        assert rc == N.MQ_EINVAL
+    rc = N.lib().mq_fuse_stream(2, 1, i32(F.GATE_NAMES.index("RX")), i32(1), i32(0), i32(1), None, out, 64,
+                                (C.c_double * 64)(), 64, used)
+    assert rc == N.MQ_EINVAL
+
+
+@pytest.mark.parametrize("name", F.GATE_NAMES)
+def test_short_streams_on_both_sides_of_the_rule(name):
+    """One gate takes the Python rules, two the native ones: the same layers."""
+    k = F.ARITIES[name]
+    op = {"name": name, "wires": list(range(k)), "parameters": [0.7] * F.PARAMS.get(name, 0)}
+    for ops in ([op], [op, op]):
+        got, ref = F.fuse(ops, 3), F._fuse_python(ops, 3, True)
+        assert [L["name"] for L in got] == [L["name"] for L in ref]
+        for a, b in zip(got, ref):
+            _same(a, b)
