@@ -75,7 +75,6 @@ __global__ void k_block_sums(Src src, uint32_t bs, uint32_t nb, double* __restri
 // are chunk bits).  27 qubits, 9 selected: 304 us with one warp per chunk and
 // table look-ups for every address, 168 us this way (6.4 TB/s).
 struct ChunkParams {
-  uint32_t nc;       // chunks
   uint8_t nb, cb;    // bits of j, bits of a chunk (cs = 2^cb)
   uint8_t spos[4];   // j bit positions (all >= max(cb, 5)) of the sibling qubits, ascending
   uint32_t img[32];  // index bit (as a mask) of every j bit
@@ -163,7 +162,8 @@ __global__ void __launch_bounds__(256) k_chunk_sums(const V2<R>* __restrict__ st
 // long runs take a warp each, which stages kSuper entries in shared memory
 // and adds them in order (every lane alike, from broadcast reads); runs of at
 // most 16 entries (two lines) a thread each.  512 runs of 256 entries: 22 us
-// by one thread per run, 4.8 us by warps.
+// by one thread per run, 4.8 us by warps; 65536 runs of two (27 qubits, 16
+// selected): a call of 282 us by warps, 260 by threads.
 constexpr int kSeqWarps = 4;
 __global__ void __launch_bounds__(32 * kSeqWarps) k_seq_sums_warp(const double* __restrict__ in, uint32_t group_len,
                                                                   uint32_t run_len, uint32_t runs_per_group,
@@ -597,7 +597,8 @@ __global__ void __launch_bounds__(kZThreads) k_pauli_z(const V2<R>* __restrict__
 // every word there (two products per pair).  Sums per word and thread stay in
 // shared memory.  Bound by the float64 work (16 products per 16 amplitudes
 // and word) and the float32 -> float64 conversions of every window; 25
-// qubits, 25 X words: 25 passes of 135 us before, three of 79 us on average now (117 with every word through the switch).
+// qubits, 25 X words: 25 passes of 135 us before, three of 79 us on average now
+// (117 with every word through the switch).
 constexpr int kTileWords = 24;
 constexpr int kTileWins = 6;
 constexpr int kPauliLT = 7;
@@ -819,7 +820,7 @@ static void launch_chunks(mq_state* h, const ChunkParams& P, double* D) {
 
 static int launch_seq(mq_state* h, const double* in, uint32_t group_len, uint32_t run_len, uint32_t runs_per_group,
                       uint32_t n_runs, double* out) {
-  if (run_len > 16)
+  if (std::min(run_len, group_len) > 16)  // a run ends with its group
     k_seq_sums_warp<<<grid_for(n_runs, kSeqWarps), 32 * kSeqWarps, 0, h->stream>>>(in, group_len, run_len,
                                                                                    runs_per_group, n_runs, out);
   else
@@ -847,7 +848,6 @@ static int marginal_device(mq_state* h, const int32_t* wires, int k, double* wor
   const uint32_t ncb = (uint32_t)(bucket_len / cs);      // chunks per bucket
   const uint32_t nsb = (ncb + kSuper - 1) / kSuper;       // super-chunks per bucket
   const uint32_t nbk = 1u << k;
-  P.nc = nc;
   P.nb = (uint8_t)n;
   while ((1u << P.cb) < cs) ++P.cb;
   // siblings: selected qubits on index bits 0-3, outside the bits of a warp
