@@ -49,6 +49,16 @@ __device__ __forceinline__ float2 caxmy(float t, float2 y, float2 x) {
   return __ffma2_rn(make_float2(t, t), y, make_float2(-x.x, -x.y));
 }
 
+// |a|^2 in float64, explicitly rounded (exact products for complex64)
+template <typename R>
+__device__ __forceinline__ double amp2(V2<R> a) {
+  const double re = (double)a.x, im = (double)a.y;
+  return __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im));
+}
+
+// Blocks of bs threads for this many threads.
+inline uint32_t grid_for(uint64_t threads, int bs) { return threads ? (uint32_t)((threads + bs - 1) / bs) : 1u; }
+
 // ---------------------------------------------------------------- async copies
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
