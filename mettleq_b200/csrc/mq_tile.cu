@@ -169,12 +169,14 @@ struct FusedParams : TileParams {
 // lmap: the transform's wires are not one run of index bits.  The twiddles
 // then read the ladder value L itself (wire j of k has weight 2^(k-1-j), other
 // bits none) instead of a shifted index: PhaseDesc g_reg / g_grp hold weights,
-// and L of a tile's base is the XOR of ltab[256 i + byte i of the tile number].
+// and L of a tile's base is the XOR of ltab[16 i + nibble i of the tile number].
+// (Every QFT launch carries the tables: by bytes, 4 KB of them, a 20-qubit
+// transform of a run took 28.4 us a call, 25.1 without.)
 struct QftParams : TileParams {
   alignas(16) float2 twf[kMaxOps][32];
   alignas(16) double2 twd[kMaxOps][32];
   uint32_t lmap;
-  uint32_t ltab[1024];
+  uint32_t ltab[128];
 };
 static_assert(sizeof(QftParams) <= 32000, "kernel parameter block too large");
 static_assert(sizeof(FusedParams) <= 32000, "kernel parameter block too large");
@@ -817,9 +819,11 @@ k_tile(const V2<R>* src, V2<R>* dst, const __grid_constant__ PT P) {
     // what a group's global index starts from: the base, or its ladder value
     uint32_t gbase = base;
     if constexpr (QFT) {
-      if (P.lmap)
-        gbase = P.ltab[tile & 255u] ^ P.ltab[256 + ((tile >> 8) & 255u)] ^ P.ltab[512 + ((tile >> 16) & 255u)] ^
-                P.ltab[768 + (tile >> 24)];
+      if (P.lmap) {
+        gbase = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) gbase ^= P.ltab[16 * i + ((tile >> (4 * i)) & 15u)];
+      }
     }
     for (int ph = 0; ph < P.n_phases; ++ph) {
       const PhaseDesc& D = phs[ph];
@@ -1576,12 +1580,15 @@ static int run_sweep(mq_state* h, Sweep& sw, const std::vector<int>& op_phase, c
     // order.  Register bits on nibble boundaries leave the ascending order;
     // scattered ones (a QFT's ordered wires) would put two lane bits on one bank
     // bit, as index bits 1 and 4, 2 and 5 or 3 and 6 are
-    std::vector<int> grp, rest;
+    uint8_t grp[16], rest[16];
+    int n_grp = 0, n_rest = 0;
+    uint32_t in_regs = 0;
+    for (int b : regs) in_regs |= 1u << b;
     const bool wide = !c64 || regs[0] == 0;  // 16-byte accesses
     const uint32_t banks = c64 ? 0xFu : 0x7u, skip = c64 && wide ? 1u : 0u;
     uint32_t seen[4] = {};
     for (int b = 0; b < m; ++b) {
-      if (std::find(regs.begin(), regs.end(), b) != regs.end()) continue;
+      if ((in_regs >> b) & 1u) continue;
       uint32_t v = phys(1u << b) & banks & ~skip;
       for (int i = 3; i >= 0; --i)
         if ((v >> i) & 1u) {
@@ -1591,10 +1598,11 @@ static int run_sweep(mq_state* h, Sweep& sw, const std::vector<int>& op_phase, c
           }
           v ^= seen[i];
         }
-      (v ? grp : rest).push_back(b);
+      if (v) grp[n_grp++] = (uint8_t)b;
+      else rest[n_rest++] = (uint8_t)b;
     }
-    grp.insert(grp.end(), rest.begin(), rest.end());
-    for (size_t j = 0; j < grp.size(); ++j) {
+    for (int j = 0; j < n_rest; ++j) grp[n_grp++] = rest[j];
+    for (int j = 0; j < n_grp; ++j) {
       D.s_grp[j] = phys(1u << grp[j]);
       D.g_grp[j] = gword(grp[j]);
     }
@@ -1699,15 +1707,15 @@ static int run_sweep(mq_state* h, Sweep& sw, const std::vector<int>& op_phase, c
     static_cast<TileParams&>(Q) = P;
     if (sw.lmap) {
       Q.lmap = 1;
-      for (int i = 0; i < 4; ++i)
-        for (int x = 0; x < 256; ++x) {
-          const uint64_t t = (uint64_t)x << (8 * i);
+      for (int i = 0; i < 8; ++i)
+        for (int x = 0; x < 16; ++x) {
+          const uint64_t t = (uint64_t)x << (4 * i);
           if (t >= P.n_tiles) break;
           const uint32_t b = deposit_runs((uint32_t)t, P.runs);
           uint32_t v = 0;
           for (int j = 0; j < h->n; ++j)
             if ((b >> j) & 1u) v |= sw.weight[j];
-          Q.ltab[256 * i + x] = v;
+          Q.ltab[16 * i + x] = v;
         }
     }
     for (int w = 0; w < P.n_ops; ++w) {
