@@ -2091,6 +2091,32 @@ int launch_layer(mq_state* h, const double* mats, const uint8_t* active, int n_t
   return MQ_OK;
 }
 
+// Groups [j0, cnt) of consecutive QFT stages, the last of them on index bit
+// blo_all: the lowest group may reach bit 0 (tmax bits), the others hold tmax -
+// pas.
+static std::vector<std::pair<int, int>> qft_groups(int j_begin, int j_end, int blo_all, int tmax, int pas) {
+  std::vector<std::pair<int, int>> groups;
+  const int cap_hi = std::max(1, tmax - pas);
+  const int cap_lo = (blo_all < pas) ? std::max(1, tmax - blo_all) : cap_hi;
+  int n_groups = 1;
+  while (cap_lo + (n_groups - 1) * cap_hi < j_end - j_begin) ++n_groups;
+  int remaining = j_end - j_begin;
+  int j0 = j_begin;
+  for (int g = 0; g < n_groups; ++g) {
+    const int left = n_groups - g;
+    int cnt = remaining;
+    if (left > 1) {
+      cnt = std::min(cap_hi, (remaining + left - 1) / left);
+      // what stays must still fit the remaining groups
+      cnt = std::max(cnt, remaining - (cap_lo + (left - 2) * cap_hi));
+    }
+    groups.push_back({j0, cnt});
+    j0 += cnt;
+    remaining -= cnt;
+  }
+  return groups;
+}
+
 // Stages [j_begin, j_end) of the QFT on qubits [q0, q0+k), first qubit = most
 // significant logical bit (sim.py:522-563 with wires = range(q0, q0+k); a
 // single stage is qft_stage_sub of qft.py:144-181).  Forward stages run in
@@ -2102,31 +2128,8 @@ int launch_qft_stages(mq_state* h, int q0, int k, int j_begin, int j_end, int in
   const int tmax = plan_tile_max(h);
   const int pas = plan_passengers(h);
   const int lad_shift = n - q0 - k;  // index bit of the last wire
-  // stage j acts on bit b_j = n-1-q0-j.  Groups of consecutive stages: the
-  // lowest group may reach bit 0 (tmax bits), the others hold tmax - pas.
-  const int count = j_end - j_begin;
-  const int blo_all = n - 1 - q0 - (j_end - 1);
-  std::vector<std::pair<int, int>> groups;  // [j0, cnt)
-  {
-    const int cap_hi = std::max(1, tmax - pas);
-    const int cap_lo = (blo_all < pas) ? std::max(1, tmax - blo_all) : cap_hi;
-    int n_groups = 1;
-    while (cap_lo + (n_groups - 1) * cap_hi < count) ++n_groups;
-    int remaining = count;
-    int j0 = j_begin;
-    for (int g = 0; g < n_groups; ++g) {
-      const int left = n_groups - g;
-      int cnt = remaining;
-      if (left > 1) {
-        cnt = std::min(cap_hi, (remaining + left - 1) / left);
-        // what stays must still fit the remaining groups
-        cnt = std::max(cnt, remaining - (cap_lo + (left - 2) * cap_hi));
-      }
-      groups.push_back({j0, cnt});
-      j0 += cnt;
-      remaining -= cnt;
-    }
-  }
+  // stage j acts on bit b_j = n-1-q0-j
+  std::vector<std::pair<int, int>> groups = qft_groups(j_begin, j_end, n - 1 - q0 - (j_end - 1), tmax, pas);
   if (inverse) std::reverse(groups.begin(), groups.end());
   for (auto [j0, cnt] : groups) {
     std::vector<int> stages;
@@ -2166,8 +2169,14 @@ int launch_qft_stages(mq_state* h, int q0, int k, int j_begin, int j_end, int in
 // phase are those of the later wires, wherever they are (QftParams::lmap).
 // The general tiles hold the low passengers beside a sweep's scattered
 // targets, so a sweep moves runs of 2^pas amplitudes as any high sweep does.
-// Before, the wires were permuted to the top of the register and back: 15 of
-// 25 qubits, inverse: four passes, 418 us; two sweeps, 226 us this way.
+// With the wires permuted to the top of the register and back, 15 of 25 qubits
+// (inverse) were four passes, 382 us on the device; two sweeps, 240 us this way.
+//
+// Register phases are those of the contiguous transform on the top k bits of the
+// register, so each amplitude takes the same factors in the same order.  (Phases
+// padded with other bits, or of other stages, were off by up to a third more: a
+// factor's error grows with the stages its phase chains.)  A sweep takes as
+// many of them as its tile holds.
 int launch_qft_wires(mq_state* h, const int32_t* wires, int k, int inverse) {
   const int n = h->n;
   const int tmax = std::min(plan_tile_max(h), h->dtype == MQ_C64 ? 12 : 11);
@@ -2179,77 +2188,95 @@ int launch_qft_wires(mq_state* h, const int32_t* wires, int k, int inverse) {
     bits[j] = n - 1 - wires[j];
     proto.weight[bits[j]] = 1u << (k - 1 - j);
   }
-  auto tile_of = [&](int j0, int cnt) {
-    std::vector<int> t;
-    for (int b = 0; b < std::max(pas, 1); ++b) t.push_back(b);
-    for (int j = j0; j < j0 + cnt; ++j)
-      if (bits[j] >= std::max(pas, 1)) t.push_back(bits[j]);
-    return t;
+  // index bits by the order of the contiguous transform: the wires from the
+  // top, the others below in their order
+  std::vector<int> image(n);
+  {
+    int at = n - 1;
+    for (int j = 0; j < k; ++j) image[at--] = bits[j];
+    for (int b = n - 1; b >= 0; --b)
+      if (!proto.weight[b]) image[at--] = b;
+  }
+  struct Phase {
+    std::vector<int> stages, slots, regs;  // regs: index bits, slots in the order of their ladder weight
+    uint32_t mask = 0;
   };
-  // as few groups of consecutive stages as fit their tiles, evenly filled
-  // where that fits too
-  auto split = [&](int most) {
-    std::vector<std::pair<int, int>> groups;
-    for (int j0 = 0; j0 < k;) {
-      int cnt = 1;
-      while (j0 + cnt < k && cnt < most && (int)tile_of(j0, cnt + 1).size() <= tmax) ++cnt;
-      groups.push_back({j0, cnt});
-      j0 += cnt;
-    }
-    return groups;
-  };
-  auto groups = split(kMaxOps);
-  const auto even = split((k + (int)groups.size() - 1) / (int)groups.size());
-  if (even.size() == groups.size()) groups = even;
+  std::vector<Phase> phases;
+  auto groups = qft_groups(0, k, n - k, tmax, pas);
   if (inverse) std::reverse(groups.begin(), groups.end());
   for (auto [j0, cnt] : groups) {
+    std::vector<int> at, order, op_phase, op_rk;
+    for (int i = 0; i < cnt; ++i) at.push_back(n - 1 - (inverse ? j0 + cnt - 1 - i : j0 + i));
+    const std::vector<int> tile = tile_for(n, at, pas, tmax, std::max(plan_min_tile(h), 5));
+    for (int b : at) order.push_back(tile_local(tile, b));
+    Sweep sw;
+    make_phases((int)tile.size(), reg_bits(h->dtype, (int)tile.size()), order, sw, op_phase, op_rk);
+    const size_t first = phases.size();
+    phases.resize(first + sw.phases.size());
+    for (size_t p = 0; p < sw.phases.size(); ++p)
+      for (int r : sw.phases[p]) {
+        phases[first + p].regs.push_back(image[tile[r]]);
+        phases[first + p].mask |= 1u << image[tile[r]];
+      }
+    for (int i = 0; i < cnt; ++i) {
+      phases[first + op_phase[i]].stages.push_back(n - 1 - at[i]);
+      phases[first + op_phase[i]].slots.push_back(op_rk[i]);
+    }
+  }
+  // the low passengers, fewer where a phase needs the room
+  const int low = std::max(1, std::min(pas, tmax - 5));
+  // sweeps [first, last) of phases, each of at most `most` stages (or one phase)
+  auto pack = [&](int most) {
+    std::vector<std::pair<size_t, size_t>> sweeps;
+    for (size_t p = 0; p < phases.size();) {
+      uint32_t mask = (1u << low) - 1u;
+      int count = 0;
+      const size_t first = p;
+      for (; p < phases.size() && p - first < (size_t)kMaxPhases; ++p) {
+        const int more = count + (int)phases[p].stages.size();
+        if (p > first && (more > most || __builtin_popcount(mask | phases[p].mask) > tmax)) break;
+        mask |= phases[p].mask;
+        count = more;
+      }
+      sweeps.push_back({first, p});
+    }
+    return sweeps;
+  };
+  // as few as can be, evenly filled where that takes no more
+  auto sweeps = pack(kMaxOps);
+  if (sweeps.size() > 1) {
+    const auto even = pack((k + (int)sweeps.size() - 1) / (int)sweeps.size());
+    if (even.size() == sweeps.size()) sweeps = even;
+  }
+  for (auto [first, last] : sweeps) {
     Sweep sw = proto;
-    sw.tile_bits = tile_of(j0, cnt);
+    uint32_t mask = (1u << low) - 1u;
+    for (size_t p = first; p < last; ++p) mask |= phases[p].mask;
     // filled with low bits to 11 (complex64: 24 warps an SM where a 10-bit tile
     // has 16; 113 against 120 us a sweep of 25 qubits, 12 bits 115; complex128:
     // 92 against 105 us)
     const int want = std::min({n, std::max(plan_min_tile(h), 11), tmax});
-    for (int b = 0; (int)sw.tile_bits.size() < want && b < n; ++b)
-      if (std::find(sw.tile_bits.begin(), sw.tile_bits.end(), b) == sw.tile_bits.end()) sw.tile_bits.push_back(b);
-    std::sort(sw.tile_bits.begin(), sw.tile_bits.end());
-    const int m = (int)sw.tile_bits.size();
-    if (m > tmax) return fail(MQ_EINVAL, "qft tile too large");
-    const int lr = reg_bits(h->dtype, m);
-    std::vector<int> stages;
-    for (int i = 0; i < cnt; ++i) stages.push_back(inverse ? j0 + cnt - 1 - i : j0 + i);
-    // register phases of lr stages; slots in the order of their ladder weight,
-    // bits that are no ladder bit of the phase's stages (other qubits, earlier
-    // wires) above them: a pair's factor reads the slots below its own
-    std::vector<int> op_phase(cnt), op_rk(cnt);
-    for (int i = 0; i < cnt; i += lr) {
+    for (int b = 0; __builtin_popcount(mask) < want && b < n; ++b) mask |= 1u << b;
+    for (int b = 0; b < n; ++b)
+      if ((mask >> b) & 1u) sw.tile_bits.push_back(b);
+    if ((int)sw.tile_bits.size() > tmax) return fail(MQ_EINVAL, "qft tile too large");
+    std::vector<int> op_phase, op_rk;
+    for (size_t p = first; p < last; ++p) {
       std::vector<int> regs;
-      uint32_t top = 0;
-      for (int j = i; j < std::min(cnt, i + lr); ++j) {
-        regs.push_back(tile_local(sw.tile_bits, bits[stages[j]]));
-        top = std::max(top, sw.weight[bits[stages[j]]]);
-      }
-      auto key = [&](int b) {
-        const uint32_t w = sw.weight[sw.tile_bits[b]];
-        return w ? (uint64_t)w : (uint64_t(1) << 40) + (uint32_t)b;
-      };
-      for (int pass = 0; pass < 2; ++pass)  // padding above the stages first
-        for (int b = m - 1; (int)regs.size() < lr && b >= 0; --b)
-          if (std::find(regs.begin(), regs.end(), b) == regs.end() && (pass || key(b) > top)) regs.push_back(b);
-      std::sort(regs.begin(), regs.end(), [&](int a, int b) { return key(a) < key(b); });
-      for (int j = i; j < std::min(cnt, i + lr); ++j) {
-        op_phase[j] = (int)sw.phases.size();
-        op_rk[j] = (int)(std::find(regs.begin(), regs.end(), tile_local(sw.tile_bits, bits[stages[j]])) - regs.begin());
+      for (int b : phases[p].regs) regs.push_back(tile_local(sw.tile_bits, b));
+      for (size_t i = 0; i < phases[p].stages.size(); ++i) {
+        TileOp op;
+        std::memset(&op, 0, sizeof(op));
+        op.kind = inverse ? OP_QFT_INV : OP_QFT_FWD;
+        op.width = (uint8_t)(k - 1 - phases[p].stages[i]);
+        if (op.width) sw.need_tw = true;
+        sw.ops.push_back(op);
+        op_phase.push_back((int)sw.phases.size());
+        op_rk.push_back(phases[p].slots[i]);
       }
       sw.phases.push_back(regs);
     }
-    for (int i = 0; i < cnt; ++i) {
-      TileOp op;
-      std::memset(&op, 0, sizeof(op));
-      op.kind = inverse ? OP_QFT_INV : OP_QFT_FWD;
-      op.width = (uint8_t)(k - 1 - stages[i]);
-      if (op.width) sw.need_tw = true;
-      sw.ops.push_back(op);
-    }
+    const int cnt = (int)sw.ops.size();
     sw.scale = std::ldexp(1.0, -(cnt / 2)) * ((cnt & 1) ? 0.70710678118654752440 : 1.0);
     sw.has_scale = true;
     int rc = run_sweep(h, sw, op_phase, op_rk);
