@@ -181,7 +181,9 @@ __device__ __forceinline__ uint32_t nib_index(uint32_t tid, uint32_t r) {
 }
 
 constexpr int kSweepThreads = 256;
-constexpr int kSweepCtas = 3;  // 80 registers a thread: 4.68 ms a batch run; 4.90 with 2 CTAs, 5.51 with 4
+// 80 registers a thread; 256 circuits of 10 to 20 qubits: 4.25 ms a run, 4.47
+// with 2 CTAs (the two tile buffers leave no room for 4)
+constexpr int kSweepCtas = 3;
 
 constexpr size_t kSweepSmem = 2 * 4096 * sizeof(float2);
 
@@ -821,8 +823,8 @@ static int record_batch(mq_batch* b, float* probs, double* z0) {
 }
 
 // Most amplitudes of a group (32 MB; a wider circuit is a group of its own).
-// 256 circuits of 10 to 20 qubits on 16 lanes: 4.91 ms a run with 2^20, 4.79 with
-// 2^21, 4.68 with 2^22, 4.80 with 2^23.
+// 256 circuits of 10 to 20 qubits on 16 lanes: 4.36 ms a run with 2^20, 4.33 with
+// 2^21, 4.25 with 2^22, 4.23 with 2^23 (twice the memory).
 constexpr size_t kGroupAmps = size_t(1) << 22;
 
 // The large circuits that run one by one, all of them with a tile plan set by

@@ -1,6 +1,7 @@
 """Shared helpers for the test-suite (random states, unitaries, circuits)."""
 from __future__ import annotations
 
+import contextlib
 import math
 
 import numpy as np
@@ -59,3 +60,22 @@ def oracle_apply_terms(o, terms) -> None:
             o.apply_global_phase(t)
         else:
             raise AssertionError(kind)
+
+
+@contextlib.contextmanager
+def device_memory_left(nbytes):
+    """About ``nbytes`` of device memory free inside (whatever earlier tests left
+    for the garbage collector is gone first)."""
+    import gc
+    import torch
+    gc.collect()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = []
+    try:
+        while torch.cuda.mem_get_info()[0] > nbytes + (4 << 20):
+            held.append(torch.empty(torch.cuda.mem_get_info()[0] - nbytes, dtype=torch.uint8, device="cuda"))
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()

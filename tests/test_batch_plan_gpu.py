@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from mettleq_b200 import _native as N
-from tests.helpers import haar_u2
+from tests.helpers import device_memory_left, haar_u2
 
 pytestmark = pytest.mark.gpu
 
@@ -68,7 +68,6 @@ def test_a_plan_without_memory_leaves_the_old_one():
     two states per width and lane, 672 MB, the groups' buffers 384 MB.  With
     about 100 MB free the plan is refused; the batch then runs as if it had
     never been asked for, and takes the plan once there is room."""
-    import torch
     from mettleq_b200.batch import CircuitBatch
     ns, ds = [21, 22, 23] * 3, [2] * 9
     mats = [_mats(2, n, c) for c, n in enumerate(ns)]
@@ -79,15 +78,11 @@ def test_a_plan_without_memory_leaves_the_old_one():
             if first:
                 assert b._lib.mq_batch_set_tiles(b._h, 11, 4, 0) == N.MQ_OK
                 assert b._lib.mq_batch_set_tiles(b._h, 0, -1, 0) == N.MQ_OK
-            torch.cuda.empty_cache()
-            free = torch.cuda.mem_get_info()[0]
-            fill = torch.empty(free - (100 << 20), dtype=torch.uint8, device="cuda")
-            assert b._lib.mq_batch_set_tiles(b._h, 11, 4, 0) == N.MQ_ENOMEM
-            assert "memory" in N.last_error()
-            b.run(mats)  # the old plan is whole before the memory is back
-            z0 = b.z0()
-            del fill
-            torch.cuda.empty_cache()
+            with device_memory_left(100 << 20):
+                assert b._lib.mq_batch_set_tiles(b._h, 11, 4, 0) == N.MQ_ENOMEM
+                assert "memory" in N.last_error()
+                b.run(mats)  # the old plan is whole before the memory is back
+                z0 = b.z0()
             assert np.array_equal(z0, zref)
             for c in range(len(ns)):
                 assert np.array_equal(b.probabilities(c), ref[c])
