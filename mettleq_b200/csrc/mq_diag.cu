@@ -489,8 +489,8 @@ int plan_diag_register(mq_state* h, int n_terms, const int32_t* kinds, const int
 // 17 qubits: 5.7e-16, the tables 3.2e-16, 1.5e-16 this way; complex64 6.7e-8,
 // 5.0e-8, 4.2e-8).
 // Bound by memory: 26 qubits, a chain and a random matching (38 bonds): 515 us
-// with eight tables, 173 us this way (6.2 TB/s); 12 qubits 3.8 and 3.7 us, 22
-// qubits 47 and 12 us.
+// with eight tables, 173 us this way in a replayed graph (164 us in a stream of
+// calls, 6.5 TB/s); 12 qubits 3.8 and 3.7 us, 22 qubits 47 and 12 us.
 template <typename R> struct DiagTile;
 template <> struct DiagTile<float> { static constexpr int M = 12, CB = 1; };
 template <> struct DiagTile<double> { static constexpr int M = 11, CB = 0; };
